@@ -115,6 +115,27 @@ def lib():
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The native host side (csrc/host_module.cpp); raises if it is missing, like lib()."""
+    global _host
+    if _host is None:
+        lib()
+        import torch  # noqa: F401  (its libraries have to be loaded first)
+        try:
+            from .csrc import _host as module
+        except ImportError as e:
+            raise SmoreError("the native host module is missing or does not load (%s): build it with "
+                             "`python smore_b200/csrc/build.py`" % e)
+        from . import ext_ops
+        module.bind(SmoreError, ext_ops)
+        module.set_timer(_timer)
+        _host = module
+    return _host
+
+
 def check(rc, what):
     if rc != 0:
         msg = lib().smore_last_error()
@@ -182,6 +203,8 @@ _timer = None
 
 def set_timer(timer):
     global _timer
+    if _host is not None:
+        _host.set_timer(timer)
     _timer = timer
 
 

@@ -24,6 +24,27 @@ TWO_SM_SRC = os.path.join(HERE, "gemm_sm100_2sm.cu")
 TWO_SM_LIB = os.path.join(HERE, "libsmore_b200_2sm.so")      # optional companion: two-SM GEMM tiles
 
 
+HOST_SRC = os.path.join(HERE, "host_module.cpp")
+HOST_LIB = os.path.join(HERE, "_host.so")      # the native host side: a Python module on top of libsmore_b200.so
+
+
+def host_command():
+    """The g++ command that builds the Python module of host_module.cpp against the installed torch."""
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-Wall", "-Wno-unknown-pragmas",
+           "-DTORCH_API_INCLUDE_EXTENSION_H", "-DTORCH_EXTENSION_NAME=_host",
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI)]
+    for d in (os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+              os.path.join(CUDA_HOME, "include"), sysconfig.get_paths()["include"]):
+        cmd += ["-isystem", d]
+    return cmd + ["-I", os.path.join(ROOT, "include"), HOST_SRC, "-o", HOST_LIB + ".tmp", "-L", os.path.join(root, "lib"),
+                  "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", "-L", HERE,
+                  "-l:libsmore_b200.so", "-Wl,-rpath,$ORIGIN"]
+
+
 def sources():
     """Sources of libsmore_b200.so (the companion library's source is built on its own)."""
     return sorted(f for f in glob.glob(os.path.join(HERE, "*.cu")) if f != TWO_SM_SRC)
@@ -120,6 +141,11 @@ def build(force=False, verbose=False):
         if two_sm.wait() != 0:
             raise RuntimeError("nvcc failed on " + TWO_SM_SRC)
         os.replace(TWO_SM_LIB + ".tmp", TWO_SM_LIB)
+    if force or _newer(HOST_LIB, _local_deps(HOST_SRC) + [os.path.abspath(__file__)]):
+        cmd = host_command()
+        print("+", " ".join(cmd), flush=True)
+        subprocess.check_call(cmd)
+        os.replace(HOST_LIB + ".tmp", HOST_LIB)
     return LIB_PATH
 
 

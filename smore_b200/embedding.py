@@ -23,6 +23,7 @@ Nothing here synchronises with the host; sizes that are only known on the device
 of distinct rows) stay there.
 """
 import os
+import weakref
 
 import torch
 import torch.nn as nn
@@ -205,71 +206,6 @@ class LazyRows(object):
         return self.owner._materialize(self.lookup).view(self._shape)
 
 
-class _Lookup(object):
-    __slots__ = ("idx", "n", "name", "order", "offset", "plan", "received", "key", "n_consumers")
-
-    def __init__(self, idx, name, order):
-        self.idx = idx          # int64 [n] on the table's device
-        self.n = idx.numel()
-        self.name = name
-        self.order = order
-        self.offset = None      # position of this lookup in its plan's concatenated id list
-        self.plan = None
-        self.received = False   # a gradient producer has run for this lookup
-        self.key = None         # identity of the caller's id tensor (sharded tables with prefetch)
-        self.n_consumers = 0    # distance ops that took this lookup's rows in the forward pass
-
-
-class _StepPlan(object):
-    """De-duplicated view of the rows a group of lookups touched, plus their gradient buffer."""
-
-    def __init__(self, opt, lookups):
-        table = opt.table
-        dev = table.device
-        self.lookups = lookups
-        off = 0
-        for lk in lookups:
-            lk.offset = off
-            lk.plan = self
-            off += lk.n
-        self.n = off
-        self.idx_all = lookups[0].idx if len(lookups) == 1 else torch.cat([lk.idx for lk in lookups])
-        self.uniq = torch.empty(self.n, dtype=torch.int64, device=dev)
-        self.slot = torch.empty(self.n, dtype=torch.int32, device=dev)
-        self.counts = torch.empty(self.n, dtype=torch.int32, device=dev)
-        self.n_unique = torch.empty(2, dtype=torch.int32, device=dev)
-        self.g_rows = torch.empty(self.n, table.shape[1], dtype=table.dtype, device=dev)
-        L = _lib.lib()
-        ws = opt._unique_workspace()
-        st = _stream_ptr(dev)
-        with torch.cuda.device(dev), _lib.timed("unique_rows"):
-            _lib.check(L.smore_unique_rows(self.idx_all.data_ptr(), self.n, table.shape[0], self.uniq.data_ptr(),
-                                           self.slot.data_ptr(), self.counts.data_ptr(), self.n_unique.data_ptr(),
-                                           ws.data_ptr(), ws.numel(), st), "smore_unique_rows")
-            _lib.check(L.smore_zero_shared_rows(self.g_rows.data_ptr(), self.counts.data_ptr(),
-                                                self.n_unique.data_ptr(), self.n, table.shape[1], st),
-                       "smore_zero_shared_rows")
-
-    def slot_of(self, lookup):
-        return self.slot[lookup.offset:lookup.offset + lookup.n]
-
-
-class _EmbedLookupFunc(torch.autograd.Function):
-    """Gathered copy of table rows with the gradient routed to the optimizer
-    (embed_optimizer.py:51-66)."""
-
-    @staticmethod
-    def forward(ctx, opt, dummy, lookup):
-        ctx.opt = opt
-        ctx.lookup = lookup
-        return opt._gather_lookup(lookup)
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        ctx.opt.accumulate_grad(ctx.lookup, grad_output.contiguous(), ctx.lookup.order)
-        return None, None, None
-
-
 class EmbeddingOptimizer(object):
     """Owns the lookups of one SparseEmbedding during a training step and applies the row-wise
     update (embed_optimizer.py:69-163).  `args` needs `optim_mode` (the reference's tuple string
@@ -278,6 +214,7 @@ class EmbeddingOptimizer(object):
 
     opt_name = None
     state_names = ()
+    core = None        # native state of the step (csrc/host_module.cpp); None for a sharded table
 
     # ---- the reference's class-level hooks -------------------------------------------------
     @classmethod
@@ -303,7 +240,9 @@ class EmbeddingOptimizer(object):
     # ---- construction --------------------------------------------------------------------------
     def __init__(self, args, sp_embed, gpu_id, lazy_names=None):
         self.args = args
-        self.sparse_embed = sp_embed
+        # the module holds this object (fwd_delegate below); holding it back strongly would leave the table
+        # and its state to the cycle collector.  With share_optim_stats the state lives on the module.
+        self._sparse_embed = weakref.ref(sp_embed) if not getattr(args, "share_optim_stats", False) else (lambda: sp_embed)
         self.gpu_id = gpu_id
         if not sp_embed.embedding.is_cuda:
             raise _lib.SmoreError("the embedding table must be in GPU memory (move the module to cuda:%s first)"
@@ -328,9 +267,9 @@ class EmbeddingOptimizer(object):
             env = os.environ.get("SMORE_B200_LAZY_ROWS", "")
             lazy_names = tuple(x for x in env.split(",") if x)
         self.lazy_names = tuple(lazy_names)
-        self.step = 0
-        self._ws = None
         self._local_state = {}
+        self.core = _lib.host().RowCore(self.table, self.dummy_tensor, _lib.OPT_IDS[self.opt_name], self.squeeze,
+                                        self.opt_name == "adam" and self.squeeze and not self.share_optim_stats)
         if self.share_optim_stats:
             for name in self.state_names:
                 if not hasattr(sp_embed, name):
@@ -348,31 +287,25 @@ class EmbeddingOptimizer(object):
             return getattr(self.sparse_embed, name)
         return self._local_state[name]
 
-    def _unique_workspace(self):
-        if self._ws is None:
-            nbytes = _lib.lib().smore_unique_rows_workspace_bytes(self.table.shape[0])
-            self._ws = torch.empty(nbytes, dtype=torch.uint8, device=self.table.device)
-        return self._ws
+    def _moments(self):
+        """(first, second) state tensors of the update kernel; None where the optimizer has none."""
+        return None, None
+
+    sparse_embed = property(lambda self: self._sparse_embed())
+
+    # the step's state lives in the native core
+    step = property(lambda self: self.core.step, lambda self, v: setattr(self.core, "step", int(v)))
+    n_fwd = property(lambda self: self.core.n_fwd)
+    _plans = property(lambda self: self.core.plans)
+    _pending = property(lambda self: self.core.pending)
+    _fused_lr = property(lambda self: self.core.fused_lr)
+    _step_dev = property(lambda self: self.core.step_dev)
+    grad_list = property(lambda self: [])      # interface parity: gradients never queue up here
+    has_grad_list = property(lambda self: [lk.order for p in self.core.plans for lk in p.lookups if lk.received])
 
     # ---- per-step bookkeeping ----------------------------------------------------------------------
-    def _drop_plans(self):
-        """Forget the step's plans.  A plan and its lookups refer to each other; cutting the links
-        here lets the step's large buffers be released at once instead of at the next cycle
-        collection."""
-        for plan in getattr(self, "_plans", []):
-            for lk in plan.lookups:
-                lk.plan = None
-            plan.lookups = []
-        self._plans = []       # plans built in this step (normally one)
-
     def zero_grad(self):
-        self.n_fwd = 0
-        self._pending = []     # lookups registered since the last plan was built
-        self._drop_plans()
-        self.grad_list = []    # kept for interface parity; gradients never queue up here
-        self.has_grad_list = []
-        self._fused_lr = None          # set by announce_lr(): rows may be updated inside the backward pass
-        self._step_advanced = False    # the device-side step counter was already advanced for this step
+        self.core.zero_grad()
 
     def announce_lr(self, lr):
         """Optional, after zero_grad() and before the step's backward pass: tells the optimizer the
@@ -385,21 +318,7 @@ class EmbeddingOptimizer(object):
         already moved)."""
         if self.opt_name != "adam" or not self.squeeze:
             return
-        self._fused_lr = float(lr)
-        if getattr(self, "_step_dev", None) is not None and not self._step_advanced:
-            self._advance_device_step(lr)
-            self._step_advanced = True
-
-    def fused_update_args(self, lookup, plan):
-        """Arguments of the in-backward update for `lookup`, or None when it does not apply."""
-        if getattr(self, "_fused_lr", None) is None or lookup.n_consumers != 1 or lookup.received:
-            return None
-        if len(self._plans) != 1 or plan is not self._plans[0] or self.share_optim_stats:
-            return None
-        dev_step = getattr(self, "_step_dev", None) is not None
-        return {"m": self.state("state_sum_fo"), "v": self.state("state_sum_sq"), "uniq": plan.uniq,
-                "lr": self._fused_lr, "step": 1 if dev_step else int(self.step) + 1,
-                "step_scalars": self._step_scalars if dev_step else None}
+        self.core.announce(float(lr), *self._moments())
 
     def _device_indices(self, indices):
         idx = indices.reshape(-1)
@@ -409,40 +328,27 @@ class EmbeddingOptimizer(object):
             idx = idx.to(self.table.device, non_blocking=True)
         return idx.contiguous()
 
-    def _gather(self, idx):
-        out = torch.empty(idx.numel(), self.table.shape[1], dtype=self.table.dtype, device=self.table.device)
-        with torch.cuda.device(self.table.device):
-            _lib.check(_lib.lib().smore_gather_rows(self.table.data_ptr(), idx.data_ptr(), self.table.shape[0],
-                                                    out.data_ptr(), idx.numel(), self.table.shape[1],
-                                                    _stream_ptr(self.table.device)), "smore_gather_rows")
-        return out
-
     def forward(self, indices, name=None):
         """What SparseEmbedding.forward delegates to (embed_optimizer.py:150-153)."""
+        core = self.core
         if indices is None:
             mat = self.table
             mat.job_handle = _DUMMY_JOB
             return mat
-        idx = self._device_indices(indices)
-        track = self.sparse_embed.training and torch.is_grad_enabled()
-        if not track:
-            out = self._gather(idx)
+        embed = self._sparse_embed()
+        if not (torch.is_grad_enabled() and (embed is None or embed.training)):
+            out = core.gather_rows(self._device_indices(indices))
             out.job_handle = _DUMMY_JOB
             return out
-        lookup = _Lookup(idx, name, self.n_fwd)
-        self.n_fwd += 1
-        self._pending.append(lookup)
+        lookup = core.lookup(indices, name)
         if name is not None and name in self.lazy_names:
             return LazyRows(self, lookup, (lookup.n, self.table.shape[1]))
-        out = _EmbedLookupFunc.apply(self, self.dummy_tensor, lookup)
+        out = core.lookup_tensor(lookup)
         out.job_handle = _DUMMY_JOB
         return out
 
     def _materialize(self, lookup):
-        return _EmbedLookupFunc.apply(self, self.dummy_tensor, lookup)
-
-    def _gather_lookup(self, lookup):
-        return self._gather(lookup.idx)
+        return self.core.lookup_tensor(lookup)
 
     def rows_operands(self, lookup):
         """(rows tensor, int64 row ids into it) that the distance kernels read for `lookup`."""
@@ -450,28 +356,13 @@ class EmbeddingOptimizer(object):
 
     def plan_for(self, lookup):
         """The step plan that covers `lookup`, built on first use from every lookup made so far."""
-        if lookup.plan is None:
-            self._plans.append(_StepPlan(self, self._pending))
-            self._pending = []
-        return lookup.plan
+        return self.core.plan_for(lookup)
 
     def accumulate_grad(self, lookup, grad_submat, fwd_idx=None):
         """Add a dense [n, width] gradient block of one lookup (embed_optimizer.py:146-148)."""
-        plan = self.plan_for(lookup)
-        # a second producer for the same positions must add to what the first one stored
-        counts_ptr = None if lookup.received else plan.counts.data_ptr()
-        lookup.received = True
-        self.has_grad_list.append(lookup.order)
-        with torch.cuda.device(self.table.device):
-            _lib.check(_lib.lib().smore_scatter_add_rows(grad_submat.data_ptr(), plan.slot_of(lookup).data_ptr(),
-                                                         counts_ptr, plan.g_rows.data_ptr(), lookup.n,
-                                                         self.table.shape[1], _stream_ptr(self.table.device)),
-                       "smore_scatter_add_rows")
+        self.core.accumulate_grad(lookup, grad_submat)
 
     # ---- the update ------------------------------------------------------------------------------
-    def _launch_update(self, uniq, g_rows, n_unique, capacity, lr):
-        raise NotImplementedError
-
     def check_status(self):
         """Raise if a kernel of this process reported trouble since the last check: a bounded wait on
         an asynchronous copy that ran out (results of that launch are invalid) or a row id outside the
@@ -496,42 +387,14 @@ class EmbeddingOptimizer(object):
         """Keep the optimizer's step counter on the device from now on (it starts from the current
         host-side value).  Needed when training steps are captured in a CUDA graph and replayed:
         Python does not run during a replay, so the bias corrections must come from device memory."""
-        dev = self.table.device
-        self._step_dev = torch.tensor([int(self.step)], dtype=torch.int64, device=dev)
-        self._step_scalars = torch.zeros(2, dtype=torch.float32, device=dev)
-
-    def _advance_device_step(self, lr):
-        dev = self.table.device
-        with torch.cuda.device(dev):
-            _lib.check(_lib.lib().smore_adam_step_scalars(self._step_dev.data_ptr(), float(lr), 0.9, 0.999,
-                                                          self._step_scalars.data_ptr(), _stream_ptr(dev)),
-                       "smore_adam_step_scalars")
-
-    def _run_update(self, opt_name, m, v, uniq, g_rows, n_unique, capacity, lr):
-        dev = self.table.device
-        if getattr(self, "_step_dev", None) is not None:
-            if not getattr(self, "_step_advanced", False):
-                self._advance_device_step(lr)
-            with torch.cuda.device(dev), _lib.timed("sparse_update_rows"):
-                _lib.check(_lib.lib().smore_sparse_update_rows_dev(
-                    _lib.OPT_IDS[opt_name], self.table.data_ptr(), None if m is None else m.data_ptr(),
-                    None if v is None else v.data_ptr(), uniq.data_ptr(), g_rows.data_ptr(), n_unique.data_ptr(),
-                    capacity, self.table.shape[1], float(lr), 0.9, 0.999, eps, self._step_scalars.data_ptr(),
-                    int(self.squeeze), _stream_ptr(dev)), "smore_sparse_update_rows_dev")
-            return
-        with torch.cuda.device(dev), _lib.timed("sparse_update_rows"):
-            _lib.check(_lib.lib().smore_sparse_update_rows(
-                _lib.OPT_IDS[opt_name], self.table.data_ptr(), None if m is None else m.data_ptr(),
-                None if v is None else v.data_ptr(), uniq.data_ptr(), g_rows.data_ptr(), n_unique.data_ptr(),
-                capacity, self.table.shape[1], float(lr), 0.9, 0.999, eps, int(self.step),
-                int(self.squeeze), _stream_ptr(dev)), "smore_sparse_update_rows")
+        self.core.use_device_step()
 
     def _merge_plans(self):
         """More than one plan in a step (lookups made after a backward had already run): fold
         them into one by treating each plan's (rows, gradients) as a dense block."""
-        plans = self._plans
+        plans = self.core.plans
         dev = self.table.device
-        lookups, blocks = [], []
+        blocks = []
         for p in plans:
             ids = p.uniq.clone()
             nu = p.n_unique[0]
@@ -539,17 +402,10 @@ class EmbeddingOptimizer(object):
             untouched = self._untouched_mask(p)
             if untouched is not None:
                 ids[untouched] = -1
-            lk = _Lookup(ids, None, -1)
-            lookups.append(lk)
-            blocks.append(p.g_rows)
-        merged = _StepPlan(self, lookups)
-        for lk, g in zip(lookups, blocks):
-            lk.received = True
-            with torch.cuda.device(dev):
-                _lib.check(_lib.lib().smore_scatter_add_rows(g.data_ptr(), merged.slot_of(lk).data_ptr(),
-                                                             merged.counts.data_ptr(), merged.g_rows.data_ptr(),
-                                                             lk.n, self.table.shape[1], _stream_ptr(dev)),
-                           "smore_scatter_add_rows")
+            blocks.append(ids)
+        merged = self.core.merged_plan(blocks)
+        for lk, p in zip(merged.lookups, plans):
+            self.core.accumulate_grad(lk, p.g_rows)
         return merged
 
     def _untouched_mask(self, plan):
@@ -567,40 +423,43 @@ class EmbeddingOptimizer(object):
 
     def apply_grad(self, lr):
         """embed_optimizer.py:155-163: the step counter advances even when nothing was looked up."""
-        self.step += 1
-        if getattr(self, "_fused_lr", None) is not None and float(lr) != self._fused_lr:
+        core = self.core
+        core.step += 1
+        fused_lr = core.fused_lr
+        if fused_lr is not None and float(lr) != fused_lr:
             raise _lib.SmoreError("apply_grad(%r) after announce_lr(%r): rows updated inside the backward pass "
-                                  "used the announced value" % (lr, self._fused_lr))
-        if not self._plans:
-            self._pending = []
-            if getattr(self, "_step_dev", None) is not None and not getattr(self, "_step_advanced", False):
-                self._advance_device_step(lr)
+                                  "used the announced value" % (lr, fused_lr))
+        m, v = self._moments()
+        if _lib._timer is not None and len(core.plans) == 1:
+            _lib.note("n_unique", core.plans[0].n_unique[0])
+        if core.apply_single_plan(float(lr), m, v):
             return
-        plan = self._plans[0] if len(self._plans) == 1 else self._merge_plans()
-        uniq = plan.uniq
-        untouched = self._untouched_mask(plan) if len(self._plans) == 1 else None
+        plans = core.plans
+        if not plans:
+            core.advance_device_step(float(lr))
+            core.end_step()
+            return
+        plan = plans[0] if len(plans) == 1 else self._merge_plans()
+        untouched = self._untouched_mask(plan) if len(plans) == 1 else None
         if untouched is not None:
-            # point untouched rows' update at nothing: give them a zero gradient and skip them by
-            # marking the row id negative is not possible for the kernel, so they are compacted out
-            keep = ~untouched & (torch.arange(plan.n, device=uniq.device) < plan.n_unique[0])
+            # rows without a gradient are compacted out of the list
+            keep = ~untouched & (torch.arange(plan.n, device=plan.uniq.device) < plan.n_unique[0])
             sel = keep.nonzero().view(-1)
-            uniq = plan.uniq[sel].contiguous()
-            g_rows = plan.g_rows[sel].contiguous()
-            n_unique = torch.tensor([sel.numel(), 0], dtype=torch.int32, device=uniq.device)
-            self._launch_update(uniq, g_rows, n_unique, sel.numel(), lr)
+            self._launch_update(plan.uniq[sel].contiguous(), plan.g_rows[sel].contiguous(), sel.numel(), lr)
         else:
-            _lib.note("n_unique", plan.n_unique[0])
-            self._launch_update(uniq, plan.g_rows, plan.n_unique, plan.n, lr)
-        self._drop_plans()
-        self._pending = []
+            core.update(plan.uniq, plan.g_rows, plan.n_unique, plan.n, float(lr), m, v)
+        core.end_step()
+
+    def _launch_update(self, uniq, g_rows, n, lr):
+        n_unique = torch.tensor([n, 0], dtype=torch.int32, device=uniq.device)
+        self.core.update(uniq, g_rows, n_unique, n, float(lr), *self._moments())
 
     def update_step(self, indices, inverse_indices, grad, lr):
         """Reference-shaped entry (embed_optimizer.py:84-86): distinct row ids + their merged gradient."""
         dev = self.table.device
         indices = indices.to(dev).contiguous()
         grad = grad.to(dev).contiguous()
-        n_unique = torch.tensor([indices.numel(), 0], dtype=torch.int32, device=dev)
-        self._launch_update(indices, grad, n_unique, indices.numel(), lr)
+        self._launch_update(indices, grad, indices.numel(), lr)
 
 
 class SGDEmbedOptimizer(EmbeddingOptimizer):
@@ -610,9 +469,6 @@ class SGDEmbedOptimizer(EmbeddingOptimizer):
     @classmethod
     def prepare_embed(cls, args, optim_mode, embed, fn_register):
         pass
-
-    def _launch_update(self, uniq, g_rows, n_unique, capacity, lr):
-        self._run_update("sgd", None, None, uniq, g_rows, n_unique, capacity, lr)
 
 
 class AdamEmbedOptimizer(EmbeddingOptimizer):
@@ -628,9 +484,8 @@ class AdamEmbedOptimizer(EmbeddingOptimizer):
         else:
             fn_register("state_sum_sq", torch.zeros(embed.embedding.size(), device=dev))
 
-    def _launch_update(self, uniq, g_rows, n_unique, capacity, lr):
-        self._run_update("adam", self.state("state_sum_fo"), self.state("state_sum_sq"), uniq, g_rows, n_unique,
-                         capacity, lr)
+    def _moments(self):
+        return self.state("state_sum_fo"), self.state("state_sum_sq")
 
 
 class AdaGradEmbedOptimizer(EmbeddingOptimizer):
@@ -645,8 +500,8 @@ class AdaGradEmbedOptimizer(EmbeddingOptimizer):
         else:
             fn_register("state_sum", torch.zeros(embed.embedding.size(), device=dev))
 
-    def _launch_update(self, uniq, g_rows, n_unique, capacity, lr):
-        self._run_update("adagrad", None, self.state("state_sum"), uniq, g_rows, n_unique, capacity, lr)
+    def _moments(self):
+        return None, self.state("state_sum")
 
 
 def get_optim_class(args):

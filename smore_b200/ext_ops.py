@@ -16,93 +16,16 @@ backward pass adds the row gradients into the owning optimizer's per-step buffer
 import torch
 
 from . import _lib
-from . import extlib_cuda as extlib
 from .embedding import LazyRows
 
 __all__ = ["l1_dist", "l2_dist", "box_dist_in", "box_dist_out", "box_dist_both", "rotate_dist", "complex_sim",
            "distmult_sim"]
 
 
-def _out_shape(entity_shape, query_shape):
-    return max(entity_shape[0], query_shape[0]), max(entity_shape[1], query_shape[1])
-
-
 def _check_broadcast(entity_shape, query_shape):
     for a, b in ((entity_shape[0], query_shape[0]), (entity_shape[1], query_shape[1])):
         if a % b != 0 and b % a != 0:
             raise ValueError("entity %s and query %s do not broadcast" % (tuple(entity_shape), tuple(query_shape)))
-
-
-class _DistFunc(torch.autograd.Function):
-    """One distance on materialised operands (the pattern of l1_dist.py:21-46 / box_dist.py:21-47)."""
-
-    @staticmethod
-    def forward(ctx, name, entity, first, second):
-        _check_broadcast(entity.shape, first.shape)
-        entity, first = entity.contiguous(), first.contiguous()
-        second = None if second is None else second.contiguous()
-        dst = torch.empty(_out_shape(entity.shape, first.shape), dtype=entity.dtype, device=entity.device)
-        extlib.dist_forward(name, entity, first, second, dst)
-        ctx.name = name
-        ctx.two = second is not None
-        if ctx.two:
-            ctx.save_for_backward(entity, first, second)
-        else:
-            ctx.save_for_backward(entity, first)
-        return dst
-
-    @staticmethod
-    def backward(ctx, grad_out):
-        if ctx.two:
-            entity, first, second = ctx.saved_tensors
-        else:
-            entity, first = ctx.saved_tensors
-            second = None
-        grad_out = grad_out.contiguous()
-        # the kernels write every element, so the buffers need not be cleared first
-        g_entity = torch.empty_like(entity)
-        g_first = torch.empty_like(first)
-        g_second = torch.empty_like(second) if ctx.two else None
-        extlib.dist_backward(ctx.name, grad_out, entity, first, second, g_entity, g_first, g_second)
-        return None, g_entity, g_first, g_second
-
-
-class _BoxBothFunc(torch.autograd.Function):
-    """Both box distances of materialised operands in one pass over the entity rows."""
-
-    @staticmethod
-    def forward(ctx, entity, center, offset):
-        _check_broadcast(entity.shape, center.shape)
-        entity, center, offset = entity.contiguous(), center.contiguous(), offset.contiguous()
-        bsize, num = _out_shape(entity.shape, center.shape)
-        d_out = torch.empty(bsize, num, dtype=entity.dtype, device=entity.device)
-        d_in = torch.empty_like(d_out)
-        L = _lib.lib()
-        with torch.cuda.device(entity.device):
-            _lib.check(L.smore_box_forward(entity.data_ptr(), None, 0, center.data_ptr(), offset.data_ptr(),
-                                           d_out.data_ptr(), d_in.data_ptr(), bsize, num, entity.shape[0],
-                                           entity.shape[1], center.shape[0], center.shape[1], center.shape[2],
-                                           torch.cuda.current_stream(entity.device).cuda_stream),
-                       "smore_box_forward")
-        ctx.save_for_backward(entity, center, offset)
-        return d_out, d_in
-
-    @staticmethod
-    def backward(ctx, g_out, g_in):
-        entity, center, offset = ctx.saved_tensors
-        g_out, g_in = g_out.contiguous(), g_in.contiguous()
-        g_entity, g_center, g_offset = torch.empty_like(entity), torch.empty_like(center), torch.empty_like(offset)
-        bsize, num = g_out.shape
-        L = _lib.lib()
-        with torch.cuda.device(entity.device):
-            _lib.check(L.smore_box_backward(g_out.data_ptr(), g_in.data_ptr(), entity.data_ptr(), None, 0,
-                                            center.data_ptr(), offset.data_ptr(), g_entity.data_ptr(), None, None,
-                                            None, g_center.data_ptr(), g_offset.data_ptr(), bsize, num,
-                                            entity.shape[0], entity.shape[1], center.shape[0], center.shape[1],
-                                            center.shape[2],
-                                            torch.cuda.current_stream(entity.device).cuda_stream),
-                       "smore_box_backward")
-        return g_entity, g_center, g_offset
 
 
 def _check_rows_operands(name, rows, first, second):
@@ -121,35 +44,17 @@ def _check_rows_operands(name, rows, first, second):
     return be, ne
 
 
-def _fused_backward(name_or_id, owner, lookup, plan, table, row_ids, first, second, gouts, g_first, g_second, branches,
-                    bsize, num, dim):
-    """Backward with the Adam step of single-contributor rows folded in, when the owning optimizer
-    announced its learning rate for this step and the shape is covered.  True when it ran."""
-    fn = getattr(owner, "fused_update_args", None)
-    fu = fn(lookup, plan) if fn is not None else None
-    if fu is None:
-        return False
-    L = _lib.lib()
-    dist_id = name_or_id if isinstance(name_or_id, int) else (
-        _lib.BOX_BOTH_ID if name_or_id == "box_both" else _lib.DIST_IDS[name_or_id])
+def _fused_backward(launch):
+    """Backward pass with the Adam step of single-contributor rows folded in, for an optimizer that
+    announced its learning rate for this step.  True when it ran, False when the shape is not covered."""
     if _lib._timer is not None:
-        _lib.note("n_single", (plan.counts == 1).sum())
-    rc = L.smore_rows_backward_fused_adam(
-        dist_id, gouts[0].data_ptr(), gouts[1].data_ptr() if len(gouts) > 1 else None, table.data_ptr(),
-        row_ids.data_ptr(), table.shape[0], first.data_ptr(), None if second is None else second.data_ptr(),
-        plan.slot_of(lookup).data_ptr(), plan.counts.data_ptr(), plan.g_rows.data_ptr(), g_first.data_ptr(),
-        None if g_second is None else g_second.data_ptr(), branches, bsize, num, dim, fu["m"].data_ptr(),
-        fu["v"].data_ptr(), fu["uniq"].data_ptr(), fu["lr"], 0.9, 0.999, 1e-8, fu["step"],
-        None if fu["step_scalars"] is None else fu["step_scalars"].data_ptr(),
-        torch.cuda.current_stream(table.device).cuda_stream)
-    if rc == -2:          # SMORE_ERR_BAD_SHAPE: not covered, nothing was enqueued
-        return False
-    _lib.check(rc, "smore_rows_backward_fused_adam")
-    return True
+        _lib.note("n_single", (launch.counts == 1).sum())
+    return launch.run()
 
 
 class _RowsDistFunc(torch.autograd.Function):
-    """A distance whose entity operand is table rows named by index.  `dummy` is the owning
+    """A distance whose entity operand is rows of a sharded table (an unsharded one takes the native
+    _host.rows_dist), named by index into the step's staged rows.  `dummy` is the owning
     optimizer's one-element parameter: it makes autograd call backward even when no query
     operand needs a gradient (the same device the reference uses, embed_optimizer.py:128,153)."""
 
@@ -206,12 +111,6 @@ class _RowsDistFunc(torch.autograd.Function):
         L = _lib.lib()
         st = torch.cuda.current_stream(table.device).cuda_stream
         bsize, num, be, ne, bc, nc, dim = ctx.sizes
-        if be == bsize and ne == num and bc == bsize and nc == 1 and num >= 16:
-            with torch.cuda.device(table.device), _lib.timed("rows_backward"):
-                if _fused_backward(ctx.name, owner, lookup, plan, table, row_ids, first, second, gouts, g_first,
-                                   g_second, 1, bsize, num, dim):
-                    lookup.received = True
-                    return None, None, None, g_first, g_second
         counts_ptr = None if lookup.received else plan.counts.data_ptr()
         lookup.received = True
         slot = plan.slot_of(lookup)
@@ -278,11 +177,6 @@ class _RowsUnionFunc(torch.autograd.Function):
         g_second = torch.empty_like(second) if ctx.two else None
         gouts = [g.contiguous() for g in gouts]
         U, B, num, dim = ctx.sizes
-        with torch.cuda.device(table.device), _lib.timed("rows_backward_union"):
-            if _fused_backward(ctx.dist_id, owner, lookup, plan, table, row_ids, first, second, gouts, g_first,
-                               g_second, U, B, num, dim):
-                lookup.received = True
-                return None, None, None, g_first, g_second
         counts_ptr = None if lookup.received else plan.counts.data_ptr()
         lookup.received = True
         slot = plan.slot_of(lookup)
@@ -324,109 +218,60 @@ def dot_precision():
     return mode
 
 
-_dot_workspaces = {}     # (device, stream) -> uint8 scratch tensor, grown on demand
+def _dot_mode(name):
+    """Precision number of the tensor-core route for `name`, -1 where it is not taken."""
+    return _DOT_PRECISIONS.get(dot_precision(), -1) if name in ("distmult", "complex") else -1
 
 
-def _dot_workspace(device, nbytes):
-    """Scratch for the GEMM route, kept per (device, stream): calls on one stream are ordered, so
-    they can share it, and nothing is allocated in the steady state."""
-    key = (device, torch.cuda.current_stream(device).cuda_stream)
-    ws = _dot_workspaces.get(key)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device)
-        _dot_workspaces[key] = ws
-    return ws
+def _dist_id(name):
+    return _lib.BOX_BOTH_ID if name == "box_both" else _lib.DIST_IDS[name]
 
 
-class _DotSharedFunc(torch.autograd.Function):
-    """score[B, K] = query[B, W] . cand[K, W]^T and its two gradients as tensor-core GEMMs."""
-
-    @staticmethod
-    def forward(ctx, cand, query, precision):
-        cand, query = cand.contiguous(), query.contiguous()
-        K, W = cand.shape[-2], cand.shape[-1]
-        B = query.shape[0]
-        L = _lib.lib()
-        dst = torch.empty(B, K, dtype=torch.float32, device=cand.device)
-        ws = _dot_workspace(cand.device, L.smore_dot_workspace_bytes(B, K, W, precision))
-        with torch.cuda.device(cand.device), _lib.timed("dot_forward"):
-            _lib.check(L.smore_dot_forward_shared(cand.data_ptr(), query.data_ptr(), dst.data_ptr(), B, K, W, precision,
-                                                  ws.data_ptr(), ws.numel(),
-                                                  torch.cuda.current_stream(cand.device).cuda_stream),
-                       "smore_dot_forward_shared")
-        ctx.save_for_backward(cand, query)
-        ctx.precision = precision
-        return dst
-
-    @staticmethod
-    def backward(ctx, gout):
-        cand, query = ctx.saved_tensors
-        gout = gout.contiguous()
-        K, W = cand.shape[-2], cand.shape[-1]
-        B = query.shape[0]
-        L = _lib.lib()
-        g_cand, g_query = torch.empty_like(cand), torch.empty_like(query)
-        ws = _dot_workspace(cand.device, L.smore_dot_workspace_bytes(B, K, W, ctx.precision))
-        with torch.cuda.device(cand.device), _lib.timed("dot_backward"):
-            _lib.check(L.smore_dot_backward_shared(gout.data_ptr(), cand.data_ptr(), query.data_ptr(), g_cand.data_ptr(),
-                                                   g_query.data_ptr(), B, K, W, ctx.precision, ws.data_ptr(), ws.numel(),
-                                                   torch.cuda.current_stream(cand.device).cuda_stream),
-                       "smore_dot_backward_shared")
-        return g_cand, g_query, None
-
-
-def _dot_shared(name, entity, first, second):
-    """The GEMM route for DistMult / ComplEx against shared candidates, or None if it does not apply."""
-    if name not in ("distmult", "complex") or first.dim() != 3:
-        return None
-    mode = dot_precision()
-    if mode == "off" or not _lib.lib().smore_dot_available():
-        return None
-    eshape = entity.as_3d() if isinstance(entity, LazyRows) else tuple(entity.shape)
-    B, nc, dim = first.shape
-    K, W = eshape[1], eshape[2]
-    if eshape[0] != 1 or nc != 1 or B < 128 or K < 128 or (B | K | W) & 3 or first.dtype != torch.float32:
-        return None
-    if W != _lib.ROW_PARTS[name] * dim or not first.is_cuda:
-        return None
+def _one_call(name, entity, first, second, dot):
+    """The op on operands that one call covers; None when a 4-D query operand has to be taken branch
+    by branch."""
     if isinstance(entity, LazyRows):
-        entity = entity.materialize()          # K rows only: the gathered copy is small here
-    query = first if second is None else torch.cat([first, second], dim=-1)
-    return _DotSharedFunc.apply(entity.reshape(K, W), query.reshape(B, W), _DOT_PRECISIONS[mode])
-
-
-def _apply(name, entity, first, second):
-    routed = _dot_shared(name, entity, first, second)
-    if routed is not None:
-        return routed
-    if isinstance(entity, LazyRows):
+        core = entity.owner.core
+        if core is not None:
+            be, ne, _ = entity.as_3d()
+            union = first.dim() == 4 and first.shape[1] == 2 and _union_in_one_pass(name, entity, first, second)
+            return _lib.host().rows_dist(core, entity.lookup, _dist_id(name), be, ne, first, second, union, dot)
+        if first.dim() == 4:
+            if not _union_in_one_pass(name, entity, first, second):
+                return None
+            return _RowsUnionFunc.apply(name, entity, entity.owner.dummy_tensor, first, second)
+        if dot >= 0 and entity.as_3d()[0] == 1:
+            routed = entity.materialize()      # the list's rows only: a small copy
+            return _lib.host().dense_dist(_dist_id(name), routed, first, second, dot)
         return _RowsDistFunc.apply(name, entity, entity.owner.dummy_tensor, first, second)
-    if name == "box_both":
-        return _BoxBothFunc.apply(entity, first, second)
-    return _DistFunc.apply(name, entity, first, second)
+    if name == "box_both" and entity.dtype == torch.float64:
+        return _dist("box_out", entity, first, second), _dist("box_in", entity, first, second)
+    return _lib.host().dense_dist(_dist_id(name), entity, first, second, dot)
 
 
 def _dist(name, entity, first, second=None):
-    """Front-end shared by all ops: 3-D operands, or a per-branch loop for 4-D query operands."""
+    """Front-end shared by all ops: 3-D operands, or 4-D query operands in one call where the kernels
+    cover them, else in a loop over the branches."""
     if getattr(entity, "remote", False):
         # rows of a sharded table that stay with their owners (smore_b200.sharded.RemoteRows)
         return entity.owner.remote_dist(name, entity, first, second)
-    if entity.dim() != first.dim():
-        if first.dim() != 4 or entity.dim() != 3:
-            raise ValueError("expected a 3-D entity operand with 3-D or 4-D query operands")
-        if _union_in_one_pass(name, entity, first, second):
-            return _RowsUnionFunc.apply(name, entity, entity.owner.dummy_tensor, first, second)
-        outs = []
-        for i in range(first.shape[1]):
-            f = first[:, i, :, :].contiguous()
-            s = None if second is None else second[:, i, :, :].contiguous()
-            outs.append(_apply(name, entity, f, s))
-        if name == "box_both":
-            return torch.stack([o[0] for o in outs], dim=1), torch.stack([o[1] for o in outs], dim=1)
-        return torch.stack(outs, dim=1)
+    four = first.dim() == 4
     if entity.dim() != 3:
-        raise ValueError("operands must be 3-D")
-    return _apply(name, entity, first, second)
+        raise ValueError("expected a 3-D entity operand with 3-D or 4-D query operands")
+    if not four and first.dim() != 3:
+        raise ValueError("operands must be 3-D, or the query operands 4-D")
+    dot = _dot_mode(name)
+    out = _one_call(name, entity, first, second, dot)
+    if out is not None:
+        return out
+    outs = []
+    for i in range(first.shape[1]):
+        f = first[:, i, :, :].contiguous()
+        s = None if second is None else second[:, i, :, :].contiguous()
+        outs.append(_one_call(name, entity, f, s, dot))
+    if name == "box_both":
+        return torch.stack([o[0] for o in outs], dim=1), torch.stack([o[1] for o in outs], dim=1)
+    return torch.stack(outs, dim=1)
 
 
 def l1_dist(entity_embed, center_embed):

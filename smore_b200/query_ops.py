@@ -9,47 +9,6 @@ from . import _lib
 from .embedding import LazyRows
 
 
-class _PathProjectFunc(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, start_center, start_offset, rel_table, off_table, rel_ids, relu_offset):
-        start_center = start_center.contiguous()
-        start_offset = None if start_offset is None else start_offset.contiguous()
-        B, D = start_center.shape
-        H = rel_ids.shape[1]
-        dev = start_center.device
-        center = torch.empty_like(start_center)
-        offset = torch.empty_like(start_center) if off_table is not None else None
-        ptr = lambda t: None if t is None else t.data_ptr()
-        with torch.cuda.device(dev), _lib.timed("path_project"):
-            _lib.check(_lib.lib().smore_path_project_forward(
-                start_center.data_ptr(), ptr(start_offset), rel_table.data_ptr(), ptr(off_table), rel_table.shape[0],
-                rel_ids.data_ptr(), rel_ids.stride(0), B, H, D, int(relu_offset), center.data_ptr(), ptr(offset),
-                torch.cuda.current_stream(dev).cuda_stream), "smore_path_project_forward")
-        ctx.save_for_backward(rel_ids, rel_table, off_table if off_table is not None else rel_table)
-        ctx.has_off, ctx.relu_offset, ctx.had_start_offset = off_table is not None, bool(relu_offset), start_offset is not None
-        ctx.sizes = (B, H, D)
-        if offset is None:
-            return center
-        return center, offset
-
-    @staticmethod
-    def backward(ctx, g_center, g_offset=None):
-        rel_ids, rel_table, off_table = ctx.saved_tensors
-        B, H, D = ctx.sizes
-        dev = rel_table.device
-        g_center = g_center.contiguous()
-        g_offset = g_offset.contiguous() if (ctx.has_off and g_offset is not None) else None
-        g_rel = torch.empty_like(rel_table)
-        g_off = torch.empty_like(off_table) if g_offset is not None else None
-        ptr = lambda t: None if t is None else t.data_ptr()
-        with torch.cuda.device(dev), _lib.timed("path_project_backward"):
-            _lib.check(_lib.lib().smore_path_project_backward(
-                g_center.data_ptr(), ptr(g_offset), off_table.data_ptr() if ctx.has_off else None, rel_table.shape[0],
-                rel_ids.data_ptr(), rel_ids.stride(0), B, H, D, int(ctx.relu_offset), g_rel.data_ptr(), ptr(g_off),
-                torch.cuda.current_stream(dev).cuda_stream), "smore_path_project_backward")
-        return (g_center, g_offset if ctx.had_start_offset else None, g_rel, g_off, None, None)
-
-
 def project_path(start_center, rel_table, rel_ids, start_offset=None, off_table=None, relu_offset=False):
     """All relation projections of a batch of path queries.
 
@@ -72,24 +31,19 @@ def project_path(start_center, rel_table, rel_ids, start_offset=None, off_table=
         raise ValueError("off_table must have the shape of rel_table")
     if not rel_table.is_contiguous() or (off_table is not None and not off_table.is_contiguous()):
         raise ValueError("relation tables must be contiguous")
-    return _PathProjectFunc.apply(start_center, start_offset, rel_table, off_table, rel_ids, relu_offset)
+    return _lib.host().path_embed(_lib.GEOMETRY_IDS["add"], None, None, start_center, start_offset, rel_table, off_table,
+                                  rel_ids, bool(relu_offset), 1.0)
 
 
 class _PathEmbedFunc(torch.autograd.Function):
-    """project_path for the multiplicative geometries and / or a start given as table rows."""
+    """Paths that start from staged rows of a sharded table (every other start takes the native
+    _host.path_embed)."""
 
     @staticmethod
     def forward(ctx, geometry, start, dummy, start_offset, rel_table, off_table, rel_ids, relu_offset, phase_scale):
-        lazy = isinstance(start, LazyRows)
-        if lazy:
-            owner, lookup = start.owner, start.lookup
-            rows, row_ids = owner.rows_operands(lookup)
-            B, W = lookup.n, rows.shape[1]
-            n_start = rows.shape[0]
-        else:
-            rows, row_ids = start.contiguous(), None
-            B, W = rows.shape
-            n_start = 0
+        owner, lookup = start.owner, start.lookup
+        rows, row_ids = owner.rows_operands(lookup)
+        B, W = lookup.n, rows.shape[1]
         two = geometry in ("rotate", "complex")
         D = W // 2 if two else W
         H = rel_ids.shape[1]
@@ -101,51 +55,40 @@ class _PathEmbedFunc(torch.autograd.Function):
         ptr = lambda t: None if t is None else t.data_ptr()
         with torch.cuda.device(dev), _lib.timed("path_project"):
             _lib.check(_lib.lib().smore_path_embed_forward(
-                _lib.GEOMETRY_IDS[geometry], rows.data_ptr(), ptr(row_ids), n_start, ptr(start_offset),
+                _lib.GEOMETRY_IDS[geometry], rows.data_ptr(), row_ids.data_ptr(), rows.shape[0], ptr(start_offset),
                 rel_table.data_ptr(), ptr(off_table), rel_table.shape[0], rel_ids.data_ptr(), rel_ids.stride(0), B, H, D,
                 int(relu_offset), float(phase_scale), out0.data_ptr(), ptr(out1),
                 torch.cuda.current_stream(dev).cuda_stream), "smore_path_embed_forward")
-        ctx.geometry, ctx.lazy, ctx.start = geometry, lazy, start if lazy else None
-        ctx.sizes, ctx.relu_offset, ctx.phase_scale = (B, H, D, W), bool(relu_offset), float(phase_scale)
+        ctx.geometry, ctx.start = geometry, start
+        ctx.sizes, ctx.relu_offset, ctx.phase_scale = (B, H, D), bool(relu_offset), float(phase_scale)
         ctx.has_off, ctx.had_start_offset = off_table is not None, start_offset is not None
-        keep = [rel_ids, rel_table, off_table if off_table is not None else rel_table]
-        if not lazy:
-            keep.append(rows)
-        ctx.save_for_backward(*keep)
+        ctx.save_for_backward(rel_ids, rel_table, off_table if off_table is not None else rel_table)
         return out0 if out1 is None else (out0, out1)
 
     @staticmethod
     def backward(ctx, g0, g1=None):
-        saved = ctx.saved_tensors
-        rel_ids, rel_table, off_table = saved[:3]
-        B, H, D, W = ctx.sizes
+        rel_ids, rel_table, off_table = ctx.saved_tensors
+        B, H, D = ctx.sizes
         dev = rel_table.device
         g0 = g0.contiguous()
         g1 = None if g1 is None else g1.contiguous()
         g_rel = torch.empty_like(rel_table)
         g_off = torch.empty_like(off_table) if (ctx.has_off and g1 is not None and ctx.geometry == "add") else None
         ptr = lambda t: None if t is None else t.data_ptr()
-        if ctx.lazy:
-            owner, lookup = ctx.start.owner, ctx.start.lookup
-            rows, row_ids = owner.rows_operands(lookup)
-            plan = owner.plan_for(lookup)
-            counts_ptr = None if lookup.received else plan.counts.data_ptr()
-            lookup.received = True
-            slot, g_rows, g_start, n_start = plan.slot_of(lookup), plan.g_rows, None, rows.shape[0]
-        else:
-            rows, row_ids, slot, g_rows, counts_ptr, n_start = saved[3], None, None, None, None, 0
-            g_start = torch.empty(B, W, dtype=torch.float32, device=dev) if ctx.geometry != "add" else None
+        owner, lookup = ctx.start.owner, ctx.start.lookup
+        rows, row_ids = owner.rows_operands(lookup)
+        plan = owner.plan_for(lookup)
+        counts_ptr = None if lookup.received else plan.counts.data_ptr()
+        lookup.received = True
         with torch.cuda.device(dev), _lib.timed("path_project_backward"):
             _lib.check(_lib.lib().smore_path_embed_backward(
-                _lib.GEOMETRY_IDS[ctx.geometry], g0.data_ptr(), ptr(g1), rows.data_ptr(), ptr(row_ids), n_start,
+                _lib.GEOMETRY_IDS[ctx.geometry], g0.data_ptr(), ptr(g1), rows.data_ptr(), row_ids.data_ptr(), rows.shape[0],
                 rel_table.data_ptr(), off_table.data_ptr() if ctx.has_off else None, rel_table.shape[0],
                 rel_ids.data_ptr(), rel_ids.stride(0), B, H, D, int(ctx.relu_offset), ctx.phase_scale, g_rel.data_ptr(),
-                ptr(g_off), ptr(g_start), ptr(slot), counts_ptr, ptr(g_rows),
+                ptr(g_off), None, plan.slot_of(lookup).data_ptr(), counts_ptr, plan.g_rows.data_ptr(),
                 torch.cuda.current_stream(dev).cuda_stream), "smore_path_embed_backward")
-        if not ctx.lazy and ctx.geometry == "add":
-            g_start = g0
         g_start_offset = g1 if (ctx.had_start_offset and ctx.geometry == "add") else None
-        return (None, None if ctx.lazy else g_start, None, g_start_offset, g_rel, g_off, None, None, None)
+        return None, None, None, g_start_offset, g_rel, g_off, None, None, None
 
 
 def embed_path(geometry, start, rel_table, rel_ids, start_offset=None, off_table=None, relu_offset=False,
@@ -186,6 +129,9 @@ def embed_path(geometry, start, rel_table, rel_ids, start_offset=None, off_table
         raise ValueError("off_table must have the shape of rel_table")
     if not rel_table.is_contiguous() or (off_table is not None and not off_table.is_contiguous()):
         raise ValueError("relation tables must be contiguous")
-    dummy = start.owner.dummy_tensor if lazy else None
-    return _PathEmbedFunc.apply(geometry, start, dummy, start_offset, rel_table, off_table, rel_ids, relu_offset,
-                                phase_scale)
+    if lazy and start.owner.core is None:
+        return _PathEmbedFunc.apply(geometry, start, start.owner.dummy_tensor, start_offset, rel_table, off_table, rel_ids,
+                                    relu_offset, phase_scale)
+    core, lookup, start = (start.owner.core, start.lookup, None) if lazy else (None, None, start)
+    return _lib.host().path_embed(_lib.GEOMETRY_IDS[geometry], core, lookup, start, start_offset, rel_table, off_table,
+                                  rel_ids, bool(relu_offset), float(phase_scale))

@@ -43,8 +43,7 @@ import os
 import torch
 
 from . import _lib
-from .embedding import (EmbeddingOptimizer, LazyRows, _DUMMY_JOB, _EmbedLookupFunc, _Lookup, _stream_ptr,
-                        eps)
+from .embedding import EmbeddingOptimizer, LazyRows, _DUMMY_JOB, _stream_ptr, eps
 
 MAX_PLANS = 4
 
@@ -477,6 +476,38 @@ class _ShardedPlan(object):
         return self.slot64[lookup.offset:lookup.offset + lookup.n]
 
 
+class _Lookup(object):
+    """A lookup of a sharded table (an unsharded table's lookups are native objects)."""
+    __slots__ = ("idx", "n", "name", "order", "offset", "plan", "received", "key", "n_consumers")
+
+    def __init__(self, idx, name, order):
+        self.idx = idx          # int64 [n] on the table's device
+        self.n = idx.numel()
+        self.name = name
+        self.order = order
+        self.offset = None      # position of this lookup in its plan's concatenated id list
+        self.plan = None
+        self.received = False   # a gradient producer has run for this lookup
+        self.key = None         # identity of the caller's id tensor (sharded tables with prefetch)
+        self.n_consumers = 0    # distance ops that took this lookup's rows in the forward pass
+
+
+class _EmbedLookupFunc(torch.autograd.Function):
+    """Gathered copy of a sharded table's rows with the gradient routed to the optimizer
+    (embed_optimizer.py:51-66)."""
+
+    @staticmethod
+    def forward(ctx, opt, dummy, lookup):
+        ctx.opt = opt
+        ctx.lookup = lookup
+        return opt._gather_lookup(lookup)
+
+    @staticmethod
+    def backward(ctx, grad_output):
+        ctx.opt.accumulate_grad(ctx.lookup, grad_output.contiguous(), ctx.lookup.order)
+        return None, None, None
+
+
 class RemoteRows(LazyRows):
     """Candidate rows of a sharded table that never come to this rank: a distance op on them is
     computed by the rows' owners (ShardedAdamOptimizer.remote_dist)."""
@@ -524,6 +555,11 @@ class ShardedAdamOptimizer(EmbeddingOptimizer):
 
     opt_name = "adam"
     state_names = ()
+    # the step's state of a sharded table lives on this object, not in a native core
+    step = n_fwd = 0
+    _plans = _pending = ()
+    _fused_lr = _step_dev = None
+    grad_list = has_grad_list = ()
 
     @classmethod
     def prepare_embed(cls, args, optim_mode, embed, fn_register):
@@ -611,6 +647,60 @@ class ShardedAdamOptimizer(EmbeddingOptimizer):
         self._r_g = f32(n_tot, W)
 
     # ---- lookups ----------------------------------------------------------------------------------
+    def _drop_plans(self):
+        """Forget the step's plans.  A plan and its lookups refer to each other; cutting the links
+        here lets the step's large buffers be released at once instead of at the next cycle
+        collection."""
+        for plan in self._plans:
+            for lk in plan.lookups:
+                lk.plan = None
+            plan.lookups = []
+        self._plans = []
+
+    def use_device_step(self):
+        dev = self.table.device
+        self._step_dev = torch.tensor([int(self.step)], dtype=torch.int64, device=dev)
+        self._step_scalars = torch.zeros(2, dtype=torch.float32, device=dev)
+
+    def _advance_device_step(self, lr):
+        dev = self.table.device
+        with torch.cuda.device(dev):
+            _lib.check(_lib.lib().smore_adam_step_scalars(self._step_dev.data_ptr(), float(lr), 0.9, 0.999,
+                                                          self._step_scalars.data_ptr(), _stream_ptr(dev)),
+                       "smore_adam_step_scalars")
+
+    def _run_update(self, opt_name, m, v, uniq, g_rows, n_unique, capacity, lr):
+        dev = self.table.device
+        if self._step_dev is not None:
+            if not self._step_advanced:
+                self._advance_device_step(lr)
+            with torch.cuda.device(dev), _lib.timed("sparse_update_rows"):
+                _lib.check(_lib.lib().smore_sparse_update_rows_dev(
+                    _lib.OPT_IDS[opt_name], self.table.data_ptr(), None if m is None else m.data_ptr(),
+                    None if v is None else v.data_ptr(), uniq.data_ptr(), g_rows.data_ptr(), n_unique.data_ptr(),
+                    capacity, self.table.shape[1], float(lr), 0.9, 0.999, eps, self._step_scalars.data_ptr(),
+                    int(self.squeeze), _stream_ptr(dev)), "smore_sparse_update_rows_dev")
+            return
+        with torch.cuda.device(dev), _lib.timed("sparse_update_rows"):
+            _lib.check(_lib.lib().smore_sparse_update_rows(
+                _lib.OPT_IDS[opt_name], self.table.data_ptr(), None if m is None else m.data_ptr(),
+                None if v is None else v.data_ptr(), uniq.data_ptr(), g_rows.data_ptr(), n_unique.data_ptr(),
+                capacity, self.table.shape[1], float(lr), 0.9, 0.999, eps, int(self.step),
+                int(self.squeeze), _stream_ptr(dev)), "smore_sparse_update_rows")
+
+    def accumulate_grad(self, lookup, grad_submat, fwd_idx=None):
+        """Add a dense [n, width] gradient block of one lookup (embed_optimizer.py:146-148)."""
+        plan = self.plan_for(lookup)
+        # a second producer for the same positions must add to what the first one stored
+        counts_ptr = None if lookup.received else plan.counts.data_ptr()
+        lookup.received = True
+        self.has_grad_list.append(lookup.order)
+        with torch.cuda.device(self.table.device):
+            _lib.check(_lib.lib().smore_scatter_add_rows(grad_submat.data_ptr(), plan.slot_of(lookup).data_ptr(),
+                                                         counts_ptr, plan.g_rows.data_ptr(), lookup.n,
+                                                         self.table.shape[1], _stream_ptr(self.table.device)),
+                       "smore_scatter_add_rows")
+
     def _workspace(self, which):
         if getattr(self, which) is None:
             nbytes = _lib.lib().smore_unique_rows_workspace_bytes(self.shard.n_rows_total)
@@ -763,12 +853,9 @@ class ShardedAdamOptimizer(EmbeddingOptimizer):
         """The learning rate apply_grad(lr) will get; needed before the backward pass of a remotely
         scored lookup, whose owners apply the row updates inside that pass."""
         self._fused_lr = float(lr)
-        if getattr(self, "_step_dev", None) is not None and not self._step_advanced:
+        if self._step_dev is not None and not self._step_advanced:
             self._advance_device_step(lr)
             self._step_advanced = True
-
-    def fused_update_args(self, lookup, plan):
-        return None         # staged rows are copies: nothing to update in place on the requester
 
     def remote_dist(self, name, rows, first, second):
         """name: a distance of ext_ops ("box_both" included) between `rows` (a RemoteRows handle viewed
@@ -906,7 +993,7 @@ class ShardedAdamOptimizer(EmbeddingOptimizer):
         G, Q, W, par = sh.world, spec.queries, sh.width, self.parity
         ptr = lambda t: None if t is None else t.data_ptr()
         second_all = self._r_queries[1] if op["two"] else None
-        dev_step = getattr(self, "_step_dev", None) is not None
+        dev_step = self._step_dev is not None
         if self.early_owner_plan:
             if len(self._plans) != op.get("plans_seen") or self._pending:
                 raise _lib.SmoreError("early_owner_plan: this rank looked up rows after the forward pass of the remotely "
@@ -1072,7 +1159,7 @@ class ShardedAdamOptimizer(EmbeddingOptimizer):
                     self._o_nuniq.data_ptr(), sh.dirty.data_ptr(), self._owner_ws.data_ptr(),
                     self._owner_ws.numel(), st), "smore_shard_owner_plan")
             _lib.note("n_unique_owner", self._o_nuniq[0])
-            dev_step = getattr(self, "_step_dev", None) is not None
+            dev_step = self._step_dev is not None
             if dev_step:
                 self._advance_device_step(lr)
             with _lib.timed("shard_reduce_update"):
