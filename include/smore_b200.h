@@ -383,6 +383,16 @@ SMORE_API int smore_filtered_ranks(const float* logits, size_t n_queries, size_t
                          size_t max_answers, int64_t* ranks, void* workspace, size_t workspace_bytes,
                          void* stream);
 
+/* smore_filtered_ranks for a caller that wants what train_process.py:140-141 keeps: of every query the
+ * ranks of its hard answers alone, in ascending order.  A query's hard answers are the last
+ * hard_ptr[q + 1] - hard_ptr[q] of its list; their ranks go to hard_ranks[hard_ptr[q] ...].
+ *   hard_ptr    [n_queries + 1] int64 on the device
+ *   hard_ranks  [hard_ptr[n_queries]] int64 */
+SMORE_API int smore_hard_ranks(const float* logits, size_t n_queries, size_t n_candidates,
+                     const int64_t* answer_ptr, const int64_t* answer_ids, size_t n_answers,
+                     size_t max_answers, const int64_t* hard_ptr, int64_t* hard_ranks, void* workspace,
+                     size_t workspace_bytes, void* stream);
+
 /* The evaluation step in one call: the n_queries queries are scored against every row of `table`
  * ([n_candidates, mul*dim], the whole entity table) and the filtered ranks of their answers are
  * counted from the scoring tiles directly; the [n_queries, n_candidates] logits are never written.
@@ -402,6 +412,13 @@ SMORE_API int smore_score_filtered_ranks(int dist_id, const float* table, size_t
                                const int64_t* answer_ptr, const int64_t* answer_ids, size_t n_answers,
                                size_t max_answers, int64_t* ranks, void* workspace, size_t workspace_bytes,
                                void* stream);
+/* The same with the ranks of the hard answers alone, sorted per query (see smore_hard_ranks). */
+SMORE_API int smore_score_hard_ranks(int dist_id, const float* table, size_t n_candidates, const float* first,
+                           const float* second, size_t n_queries, size_t dim, double gamma, double cen,
+                           const int64_t* answer_ptr, const int64_t* answer_ids, size_t n_answers,
+                           size_t max_answers, const int64_t* hard_ptr, int64_t* hard_ranks,
+                           void* workspace, size_t workspace_bytes, void* stream);
+
 
 /* ------------------------------------------------------------------------------------------
  * Negative sampling on the GPU (the step before the row lookups).

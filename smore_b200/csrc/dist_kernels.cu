@@ -1347,69 +1347,132 @@ __device__ __forceinline__ float logit_of(const float* acc, int kind, float gamm
   return acc[0];
 }
 
-// answer scores [Q, n_answers] (one or two distances) -> logits, in place of dst0
-template <int NOUT>
-__global__ void __launch_bounds__(256)
-    answer_logits_kernel(float* __restrict__ d0, const float* __restrict__ d1, size_t n, int kind, float gamma, float cen) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    float acc[2] = {d0[i], NOUT == 2 ? d1[i] : 0.f};
-    d0[i] = logit_of<NOUT>(acc, kind, gamma, cen);
-  }
-}
+// The answers' own logits, [n_answers] in the order of answer_ids.  A cell's terms have to be added one
+// after the other, as tile_scores does, so an answer is one thread's serial sum; the rows it reads are
+// first brought to shared memory by the whole CTA, kAnswersPerCta answers of one query at a time.
+// (960 answers of 32 queries, dim 400: 72 us when the scoring tile computed every query against every
+// answer, for the diagonal.)
+constexpr int kAnswersPerCta = 8;
+constexpr int kAnswerDims = 512;    // dims staged at a time
 
 template <class Term>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(128)
+    answer_logits_kernel(SharedArgs a, const int64_t* __restrict__ answer_ptr, int kind, float gamma, float cen,
+                         float* __restrict__ logits) {
+  __shared__ __align__(16) float q[2][kAnswerDims];
+  __shared__ __align__(16) float e[kAnswersPerCta][Term::kMul][kAnswerDims + 4];
+  const int b = blockIdx.x;
+  const long long begin = answer_ptr[b] + (long long)blockIdx.y * kAnswersPerCta;
+  const int n = (int)max(0LL, min((long long)kAnswersPerCta, answer_ptr[b + 1] - begin));
+  if (n == 0) return;
+  float acc[Term::kNOut];
+#pragma unroll
+  for (int o = 0; o < Term::kNOut; ++o) acc[o] = 0.f;
+  bool bad = false;
+  for (int d0 = 0; d0 < a.dim; d0 += kAnswerDims) {
+    const int n4 = min(kAnswerDims, a.dim - d0) >> 2;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n4; i += blockDim.x) {
+      reinterpret_cast<float4*>(q[0])[i] = __ldg(reinterpret_cast<const float4*>(a.first + (size_t)b * a.dim + d0) + i);
+      if (Term::kNQ == 2)
+        reinterpret_cast<float4*>(q[1])[i] = __ldg(reinterpret_cast<const float4*>(a.second + (size_t)b * a.dim + d0) + i);
+    }
+    for (int i = threadIdx.x; i < n * Term::kMul * n4; i += blockDim.x) {
+      const int r = i / (Term::kMul * n4), rem = i - r * Term::kMul * n4, part = rem / n4, c = rem - part * n4;
+      const long long row = max(checked_row_id(a.idx, begin + r, a.n_rows, &g_async_status), 0LL);
+      reinterpret_cast<float4*>(e[r][part])[c] =
+          __ldg(reinterpret_cast<const float4*>(a.ent + ((size_t)row * Term::kMul + part) * a.dim + d0) + c);
+    }
+    __syncthreads();
+    if (threadIdx.x < n) {
+      const int r = threadIdx.x;
+      bad = checked_row_id(a.idx, begin + r, a.n_rows, &g_async_status) < 0;
+      for (int i = 0; i < n4; ++i) {
+        const float4 e0 = reinterpret_cast<const float4*>(e[r][0])[i], e1 = reinterpret_cast<const float4*>(e[r][Term::kMul - 1])[i];
+        const float4 q0 = reinterpret_cast<const float4*>(q[0])[i];
+        const float4 q1 = Term::kNQ == 2 ? reinterpret_cast<const float4*>(q[1])[i] : q0;
+        fwd4<Term>(e0, e1, q0, q1, acc);
+      }
+    }
+  }
+  if (threadIdx.x < n) logits[begin + threadIdx.x] = bad ? NAN : logit_of<Term::kNOut>(acc, kind, gamma, cen);
+}
+
+// Scores the queries against every row of the table and counts, per answer, the candidates whose first
+// answer behind them it is.  A fixed number of CTAs walks the tiles; the answers of a CTA's queries (keys,
+// ids, counts) stay in shared memory while they fit (`cap` answers), and the counts go to `hist` once.
+// A CTA keeps one query tile (blockIdx.y) and takes candidate tiles blockIdx.x, + gridDim.x, ...
+template <class Term>
+__global__ void __launch_bounds__(kTileThreads)
     score_rank_kernel(SharedArgs a, int kind, float gamma, float cen, const int64_t* __restrict__ answer_ptr,
                       const uint32_t* __restrict__ sorted_logit, const int64_t* __restrict__ sorted_id,
-                      int32_t* __restrict__ hist) {
-  __shared__ __align__(16) TileSmem<Term> sm;
-  __shared__ long long q_begin[kTileB], q_worst_id[kTileB];
-  __shared__ int q_count[kTileB];
-  __shared__ uint32_t q_worst[kTileB];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int b0 = blockIdx.y * kTileB, k0 = blockIdx.x * kTileK;
+                      int32_t* __restrict__ hist, int cap) {
+  extern __shared__ __align__(16) unsigned char tile_smem[];
+  TileSmem<Term>& sm = *reinterpret_cast<TileSmem<Term>*>(tile_smem);
+  uint32_t* key = reinterpret_cast<uint32_t*>(tile_smem + sizeof(TileSmem<Term>));   // [cap]
+  int32_t* id = reinterpret_cast<int32_t*>(key + cap);                               // [cap]
+  int32_t* count = id + cap;                                                         // [cap]
+  __shared__ int q_at[kTileB], q_count[kTileB];       // a query's first answer, relative to the tile's; how many
+  const int tx = threadIdx.x % kTileTx, ty = threadIdx.x / kTileTx;
+  const int b0 = blockIdx.y * kTileB;
+  const long long first_answer = answer_ptr[b0];
+  const int n_tile = (int)(answer_ptr[min(a.B, b0 + kTileB)] - first_answer);
+  const bool local = n_tile <= cap;
   if (threadIdx.x < kTileB) {
     const int b = b0 + threadIdx.x;
-    long long begin = 0, wid = 0;
-    int A = 0;
-    uint32_t wk = 0;
-    if (b < a.B) {
-      begin = answer_ptr[b];
-      A = (int)(answer_ptr[b + 1] - begin);
-      if (A > 0) {
-        wk = sorted_logit[begin + A - 1];
-        wid = sorted_id[begin + A - 1];
-      }
-    }
-    q_begin[threadIdx.x] = begin;
-    q_count[threadIdx.x] = A;
-    q_worst[threadIdx.x] = wk;
-    q_worst_id[threadIdx.x] = wid;
+    q_at[threadIdx.x] = b < a.B ? (int)(answer_ptr[b] - first_answer) : 0;
+    q_count[threadIdx.x] = b < a.B ? (int)(answer_ptr[b + 1] - answer_ptr[b]) : 0;
   }
-  float acc[4][4][Term::kNOut];
-  tile_scores<Term>(a, sm, b0, k0, acc);      // (its barriers also order the writes above)
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int bl = ty * 4 + i;
-    const int A = q_count[bl];
-    if (b0 + bl >= a.B || A == 0) continue;
-    const long long begin = q_begin[bl];
-    const uint32_t worst = q_worst[bl];
-    const long long worst_id = q_worst_id[bl];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const long long e = k0 + tx * 4 + j;
-      if (e >= a.K) continue;
-      const uint32_t x = rank_key(logit_of<Term::kNOut>(acc[i][j], kind, gamma, cen));
-      if (!rank_ahead(x, e, worst, worst_id)) continue;      // ahead of no answer (the usual case)
-      int lo = 0, hi = A - 1;   // first answer this candidate is ahead of
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (rank_ahead(x, e, sorted_logit[begin + mid], sorted_id[begin + mid])) hi = mid;
-        else lo = mid + 1;
-      }
-      atomicAdd(hist + begin + lo, 1);
+  if (local) {
+    for (int i = threadIdx.x; i < n_tile; i += kTileThreads) {
+      key[i] = sorted_logit[first_answer + i];
+      id[i] = (int32_t)sorted_id[first_answer + i];
+      count[i] = 0;
     }
+  }
+  const int k_tiles = (a.K + kTileK - 1) / kTileK;
+  for (int kt = blockIdx.x; kt < k_tiles; kt += gridDim.x) {
+    float acc[kCellsB][kCellsK][Term::kNOut];
+    const int k0 = kt * kTileK;
+    tile_scores<Term>(a, sm, b0, k0, acc);      // (its barriers also order the writes above)
+#pragma unroll
+    for (int i = 0; i < kCellsB; ++i) {
+      const int bl = ty + kTileTy * i;
+      const int A = q_count[bl];
+      if (A == 0) continue;
+      const int at = q_at[bl];
+#pragma unroll
+      for (int j = 0; j < kCellsK; ++j) {
+        const int k = k0 + tx + kTileTx * j;
+        if (k >= a.K) continue;
+        const uint32_t x = rank_key(logit_of<Term::kNOut>(acc[i][j], kind, gamma, cen));
+        int lo = 0, hi = A;       // first answer this candidate is ahead of; A: it is ahead of none
+        if (local) {
+          while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (rank_ahead(x, k, key[at + mid], id[at + mid])) hi = mid;
+            else lo = mid + 1;
+          }
+          if (lo < A) atomicAdd(count + at + lo, 1);
+        } else {
+          const uint32_t* gk = sorted_logit + first_answer + at;
+          const int64_t* gi = sorted_id + first_answer + at;
+          if (!rank_ahead(x, k, gk[A - 1], gi[A - 1])) continue;
+          --hi;
+          while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (rank_ahead(x, k, gk[mid], gi[mid])) hi = mid;
+            else lo = mid + 1;
+          }
+          atomicAdd(hist + first_answer + at + lo, 1);
+        }
+      }
+    }
+  }
+  if (local) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < n_tile; i += kTileThreads)
+      if (count[i]) atomicAdd(hist + first_answer + i, count[i]);
   }
 }
 
@@ -1474,7 +1537,8 @@ static RowPlan plan_rows(const Shape& s, bool aligned) {
 static bool shared_shape(const Shape& s, bool aligned) {
   return aligned && s.be == 1 && s.bc == s.bsize && s.ne == s.num && s.nc == 1 && (s.dim & 3) == 0 &&
          s.bsize >= 8 && s.num >= 8 && s.bsize < ((size_t)1 << 24) && s.num < ((size_t)1 << 30) &&
-         s.dim < ((size_t)1 << 20) && (s.bsize + kTileB - 1) / kTileB <= 65535;   // grid.y / grid.z limits
+         s.dim < ((size_t)1 << 20) &&
+         ((s.bsize + kTileB - 1) / kTileB) * ((s.num + kTileK - 1) / kTileK) <= (size_t)INT_MAX;   // tiles: grid.x
 }
 
 // Launches row_backward_bulk_kernel when the row width suits it.  Returns 1 when launched, 0 when
@@ -1672,8 +1736,10 @@ static int launch_forward(const Shape& s, const float* ent, const int64_t* idx, 
   }
   if (shared_shape(s, aligned)) {
     SharedArgs a{ent, idx, first, second, (int)s.bsize, (int)s.num, (int)s.dim, (long long)s.n_rows};
-    dim3 grid((unsigned)((s.num + kTileK - 1) / kTileK), (unsigned)((s.bsize + kTileB - 1) / kTileB));
-    shared_forward_kernel<Term><<<grid, 256, 0, st>>>(a, dst0, dst1);
+    const unsigned grid = (unsigned)(((s.num + kTileK - 1) / kTileK) * ((s.bsize + kTileB - 1) / kTileB));
+    auto kern = shared_forward_kernel<Term>;
+    if (int rc = allow_large_smem(kern, (int)sizeof(TileSmem<Term>))) return rc;
+    kern<<<grid, kTileThreads, sizeof(TileSmem<Term>), st>>>(a, dst0, dst1);
     return check_launch("shared_forward_kernel");
   }
   CellArgs<float> a{ent, idx, first, second, s.bsize, s.num, s.be, s.ne, s.bc, s.nc, s.dim, (long long)s.n_rows};
@@ -1906,6 +1972,72 @@ static int backward_common(int id, const float* gout, const float* ent, const in
   cudaStream_t st = (cudaStream_t)stream;
   SMORE_DISPATCH(id, launch_backward<Term>(s, gout, gout, ent, idx, first, second, g_ent, slot, slot_count,
                                            g_rows, g_first, g_second, st));
+}
+
+// One call of the evaluation step; ranks of all answers, or (hard_ptr given) the sorted ranks of the hard ones.
+static int score_filtered_ranks_impl(int dist_id, const float* table, size_t n_candidates, const float* first,
+                                     const float* second, size_t n_queries, size_t dim, double gamma, double cen,
+                                     const int64_t* answer_ptr, const int64_t* answer_ids, size_t n_answers,
+                                     size_t max_answers, const int64_t* hard_ptr, int64_t* ranks, void* workspace,
+                                     size_t workspace_bytes, void* stream) {
+  if (n_queries == 0 || n_answers == 0) return SMORE_OK;
+  const bool both = dist_id == SMORE_DIST_BOX_BOTH;
+  if (!both && (dist_id < 0 || dist_id >= SMORE_DIST_COUNT))
+    return fail(SMORE_ERR_BAD_DIST, "unknown distance id %d", dist_id);
+  if (dist_id == SMORE_DIST_BOX_OUT || dist_id == SMORE_DIST_BOX_IN)
+    return fail(SMORE_ERR_BAD_DIST, "score_filtered_ranks: Query2box logits need both distances (SMORE_DIST_BOX_BOTH)");
+  const bool two = both || needs_second(dist_id);
+  if (!table || !first || (two && !second) || !answer_ptr || !answer_ids || !ranks || !workspace)
+    return fail(SMORE_ERR_NULL, "score_filtered_ranks: NULL pointer");
+  if (workspace_bytes < smore_score_filtered_ranks_workspace_bytes(n_queries, n_answers) ||
+      (reinterpret_cast<uintptr_t>(workspace) & 255))
+    return fail(SMORE_ERR_WORKSPACE, "score_filtered_ranks: workspace too small or not 256-byte aligned");
+  if (!second) second = first;
+  const Shape s_all{n_queries, n_candidates, 1, n_candidates, n_queries, 1, dim, 0};
+  if (int rc = validate_shape(s_all)) return rc;
+  const bool aligned = aligned16(table) && aligned16(first) && aligned16(second);
+  if (!shared_shape(s_all, aligned) || n_answers < 8 || max_answers == 0)
+    return fail(SMORE_ERR_BAD_SHAPE,
+                "score_filtered_ranks: needs 16-byte aligned operands, dim a multiple of 4, at least 8 queries, "
+                "8 candidates and 8 answers in all");
+  const RankWorkspace w = carve_rank_workspace(workspace, n_answers);
+  float* logits = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + w.bytes);
+  const int kind = (dist_id == SMORE_DIST_COMPLEX || dist_id == SMORE_DIST_DISTMULT) ? kLogitIdentity
+                   : dist_id == SMORE_DIST_L2 ? kLogitGammaMinusSqrt : kLogitGammaMinus;
+  cudaStream_t st = (cudaStream_t)stream;
+  SharedArgs a_ans{table, answer_ids, first, second, (int)n_queries, (int)n_answers, (int)dim, (long long)n_candidates};
+  SharedArgs a_all{table, nullptr, first, second, (int)n_queries, (int)n_candidates, (int)dim, 0};
+  const dim3 grid_ans((unsigned)n_queries, (unsigned)((max_answers + kAnswersPerCta - 1) / kAnswersPerCta));
+  const size_t q_tiles = (n_queries + kTileB - 1) / kTileB, k_tiles = (n_candidates + kTileK - 1) / kTileK;
+  // answers of a query tile kept on the SM: four CTAs per SM leave room for about a thousand (12 bytes each)
+  const int cap = 1024;
+#define SCORE_RANK(TERM)                                                                                             \
+  {                                                                                                                  \
+    answer_logits_kernel<TERM><<<grid_ans, 128, 0, st>>>(a_ans, answer_ptr, kind, (float)gamma, (float)cen, logits); \
+    count_launches(1);                                                                                               \
+    if (int rc = rank_sort_answers(logits, n_answers, answer_ptr, answer_ids, true, n_queries, n_answers,            \
+                                   max_answers, w, st))                                                              \
+      return rc;                                                                                                     \
+    const size_t smem = sizeof(TileSmem<TERM>) + (size_t)cap * 12;                                                   \
+    auto kern = score_rank_kernel<TERM>;                                                                             \
+    if (int rc = allow_large_smem(kern, (int)smem)) return rc;                                                       \
+    int per_sm = 0;                                                                                                  \
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTileThreads, smem) != cudaSuccess || per_sm < 1) \
+      per_sm = 1;                                                                                                    \
+    const size_t ctas = std::max<size_t>(1, (size_t)sm_count() * per_sm / q_tiles);                                  \
+    const dim3 grid((unsigned)std::min(ctas, k_tiles), (unsigned)q_tiles);                                           \
+    kern<<<grid, kTileThreads, smem, st>>>(a_all, kind, (float)gamma, (float)cen, answer_ptr, w.sorted_logit,        \
+                                           w.sorted_id, w.hist, cap);                                                \
+  }
+  if (both) SCORE_RANK(TermBoxBoth)
+  else if (dist_id == SMORE_DIST_ROTATE) SCORE_RANK(TermRotate)
+  else if (dist_id == SMORE_DIST_L1) SCORE_RANK(TermL1)
+  else if (dist_id == SMORE_DIST_L2) SCORE_RANK(TermL2)
+  else if (dist_id == SMORE_DIST_COMPLEX) SCORE_RANK(TermComplex)
+  else SCORE_RANK(TermDistmult)
+#undef SCORE_RANK
+  if (int rc = check_launch("score_rank_kernel")) return rc;
+  return rank_finalize(answer_ptr, w, hard_ptr, max_answers, ranks, n_queries, st);
 }
 
 }  // namespace smore
@@ -2172,8 +2304,8 @@ int smore_rows_backward_fused_adam_ragged(int dist_id, const float* gout0, const
 }
 
 size_t smore_score_filtered_ranks_workspace_bytes(size_t n_queries, size_t n_answers) {
-  const size_t scores = ((n_queries * n_answers * sizeof(float) + 255) / 256) * 256;
-  return carve_rank_workspace(nullptr, n_answers).bytes + 2 * scores + 256;
+  (void)n_queries;
+  return carve_rank_workspace(nullptr, n_answers).bytes + ((n_answers * sizeof(float) + 255) / 256) * 256 + 256;
 }
 
 int smore_score_filtered_ranks(int dist_id, const float* table, size_t n_candidates, const float* first,
@@ -2181,60 +2313,18 @@ int smore_score_filtered_ranks(int dist_id, const float* table, size_t n_candida
                                const int64_t* answer_ptr, const int64_t* answer_ids, size_t n_answers,
                                size_t max_answers, int64_t* ranks, void* workspace, size_t workspace_bytes,
                                void* stream) {
-  if (n_queries == 0 || n_answers == 0) return SMORE_OK;
-  const bool both = dist_id == SMORE_DIST_BOX_BOTH;
-  if (!both && (dist_id < 0 || dist_id >= SMORE_DIST_COUNT))
-    return fail(SMORE_ERR_BAD_DIST, "unknown distance id %d", dist_id);
-  if (dist_id == SMORE_DIST_BOX_OUT || dist_id == SMORE_DIST_BOX_IN)
-    return fail(SMORE_ERR_BAD_DIST, "score_filtered_ranks: Query2box logits need both distances (SMORE_DIST_BOX_BOTH)");
-  const bool two = both || needs_second(dist_id);
-  if (!table || !first || (two && !second) || !answer_ptr || !answer_ids || !ranks || !workspace)
-    return fail(SMORE_ERR_NULL, "score_filtered_ranks: NULL pointer");
-  if (workspace_bytes < smore_score_filtered_ranks_workspace_bytes(n_queries, n_answers) ||
-      (reinterpret_cast<uintptr_t>(workspace) & 255))
-    return fail(SMORE_ERR_WORKSPACE, "score_filtered_ranks: workspace too small or not 256-byte aligned");
-  if (!second) second = first;
-  const Shape s_all{n_queries, n_candidates, 1, n_candidates, n_queries, 1, dim, 0};
-  const Shape s_ans{n_queries, n_answers, 1, n_answers, n_queries, 1, dim, n_candidates};
-  if (int rc = validate_shape(s_all)) return rc;
-  const bool aligned = aligned16(table) && aligned16(first) && aligned16(second);
-  if (!shared_shape(s_all, aligned) || !shared_shape(s_ans, aligned) || max_answers == 0)
-    return fail(SMORE_ERR_BAD_SHAPE,
-                "score_filtered_ranks: needs 16-byte aligned operands, dim a multiple of 4, at least 8 queries, "
-                "8 candidates and 8 answers in all");
-  const RankWorkspace w = carve_rank_workspace(workspace, n_answers);
-  const size_t scores = ((n_queries * n_answers * sizeof(float) + 255) / 256) * 256;
-  float* d0 = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + w.bytes);
-  float* d1 = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + w.bytes + scores);
-  const int kind = (dist_id == SMORE_DIST_COMPLEX || dist_id == SMORE_DIST_DISTMULT) ? kLogitIdentity
-                   : dist_id == SMORE_DIST_L2 ? kLogitGammaMinusSqrt : kLogitGammaMinus;
-  cudaStream_t st = (cudaStream_t)stream;
-  SharedArgs a_ans{table, answer_ids, first, second, (int)n_queries, (int)n_answers, (int)dim, (long long)n_candidates};
-  SharedArgs a_all{table, nullptr, first, second, (int)n_queries, (int)n_candidates, (int)dim, 0};
-  dim3 grid_ans((unsigned)((n_answers + kTileK - 1) / kTileK), (unsigned)((n_queries + kTileB - 1) / kTileB));
-  dim3 grid_all((unsigned)((n_candidates + kTileK - 1) / kTileK), (unsigned)((n_queries + kTileB - 1) / kTileB));
-  const int egrid = grid_for(n_queries * n_answers, 256);
-#define SCORE_RANK(TERM)                                                                                          \
-  {                                                                                                               \
-    shared_forward_kernel<TERM><<<grid_ans, 256, 0, st>>>(a_ans, d0, d1);                                         \
-    answer_logits_kernel<TERM::kNOut><<<egrid, 256, 0, st>>>(d0, d1, n_queries * n_answers, kind, (float)gamma,  \
-                                                             (float)cen);                                         \
-    count_launches(2);                                                                                            \
-    if (int rc = rank_sort_answers(d0, n_answers, answer_ptr, answer_ids, true, n_queries, n_answers, max_answers, \
-                                   w, st))                                                                        \
-      return rc;                                                                                                  \
-    score_rank_kernel<TERM><<<grid_all, 256, 0, st>>>(a_all, kind, (float)gamma, (float)cen, answer_ptr,          \
-                                                      w.sorted_logit, w.sorted_id, w.hist);                       \
-  }
-  if (both) SCORE_RANK(TermBoxBoth)
-  else if (dist_id == SMORE_DIST_ROTATE) SCORE_RANK(TermRotate)
-  else if (dist_id == SMORE_DIST_L1) SCORE_RANK(TermL1)
-  else if (dist_id == SMORE_DIST_L2) SCORE_RANK(TermL2)
-  else if (dist_id == SMORE_DIST_COMPLEX) SCORE_RANK(TermComplex)
-  else SCORE_RANK(TermDistmult)
-#undef SCORE_RANK
-  if (int rc = check_launch("score_rank_kernel")) return rc;
-  return rank_finalize(answer_ptr, w, ranks, n_queries, st);
+  return score_filtered_ranks_impl(dist_id, table, n_candidates, first, second, n_queries, dim, gamma, cen, answer_ptr,
+                                   answer_ids, n_answers, max_answers, nullptr, ranks, workspace, workspace_bytes, stream);
+}
+
+int smore_score_hard_ranks(int dist_id, const float* table, size_t n_candidates, const float* first, const float* second,
+                           size_t n_queries, size_t dim, double gamma, double cen, const int64_t* answer_ptr,
+                           const int64_t* answer_ids, size_t n_answers, size_t max_answers, const int64_t* hard_ptr,
+                           int64_t* hard_ranks, void* workspace, size_t workspace_bytes, void* stream) {
+  if (!hard_ptr) return fail(SMORE_ERR_NULL, "score_hard_ranks: hard_ptr is NULL");
+  return score_filtered_ranks_impl(dist_id, table, n_candidates, first, second, n_queries, dim, gamma, cen, answer_ptr,
+                                   answer_ids, n_answers, max_answers, hard_ptr, hard_ranks, workspace, workspace_bytes,
+                                   stream);
 }
 
 extern "C" int smore_peer_async_status(int* status);   // peer_kernels.cu (not part of the public header)

@@ -73,10 +73,12 @@ struct TermBoxBoth {
   static constexpr int kMul = 1, kNQ = 2, kNOut = 2;
   template <typename T>
   __device__ __forceinline__ static void fwd(T e0, T, T c, T o, T* acc) {
-    T a = t_abs(e0 - c);
-    T t = a - o;
-    acc[0] += t > T(0) ? t : T(0);
-    acc[1] += t_abs(t_min(a, o));
+    // max(a - o, 0) as a - min(a, o): the same value bit for bit (the difference of equal numbers is
+    // +0), and the minimum is needed anyway: five instructions per term instead of six
+    const T a = t_abs(e0 - c);
+    const T m = t_min(a, o);
+    acc[0] += a - m;
+    acc[1] += t_abs(m);
   }
   template <typename T>
   __device__ __forceinline__ static void bwd(const T* g, T e0, T, T c, T o, T& ge0, T&, T& gc, T& go) {

@@ -832,6 +832,117 @@ py::object path_embed(int geometry, const std::shared_ptr<RowCore>& core, const 
   return py::cast(out0);
 }
 
+// ---- evaluation --------------------------------------------------------------------------------------
+// Answer lists of a batch of queries (Python iterables of ids) packed into one pinned block and sent to the
+// device with one copy: [answer_ptr (Q + 1) | hard_ptr (Q + 1) | ids].
+struct Answers {
+  std::vector<int64_t> hard_counts;
+  int64_t Q = 0, n = 0, longest = 0, n_hard = 0;
+  Tensor device;
+
+  const int64_t* ptr() const { return (const int64_t*)device.data_ptr(); }
+  const int64_t* hard_ptr() const { return ptr() + Q + 1; }
+  const int64_t* ids() const { return ptr() + 2 * (Q + 1); }
+};
+
+void append_ids(PyObject* list, int64_t limit, std::vector<int64_t>& out) {
+  py::object fast = py::reinterpret_steal<py::object>(PySequence_Fast(list, "answers must be iterables of candidate ids"));
+  if (!fast) throw py::error_already_set();
+  const Py_ssize_t n = PySequence_Fast_GET_SIZE(fast.ptr());
+  PyObject** items = PySequence_Fast_ITEMS(fast.ptr());
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    int64_t v;
+    if (PyLong_Check(items[i])) {
+      v = PyLong_AsLongLong(items[i]);
+    } else {
+      py::object num = py::reinterpret_steal<py::object>(PyNumber_Long(items[i]));
+      if (!num) throw py::error_already_set();
+      v = PyLong_AsLongLong(num.ptr());
+    }
+    if (v == -1 && PyErr_Occurred()) throw py::error_already_set();
+    if (v < 0 || v >= limit) throw py::value_error("answer ids must lie in [0, " + std::to_string(limit) + ")");
+    out.push_back(v);
+  }
+}
+
+Answers pack_answers(const py::sequence& easy, const py::sequence& hard, int64_t Q, int64_t n_candidates, const Tensor& like) {
+  if ((int64_t)py::len(easy) != Q || (int64_t)py::len(hard) != Q)
+    throw py::value_error("one easy and one hard answer list per query");
+  Answers a;
+  a.Q = Q;
+  std::vector<int64_t> ids, ptr{0}, hard_ptr{0};
+  for (int64_t q = 0; q < Q; ++q) {
+    append_ids(py::object(easy[q]).ptr(), n_candidates, ids);
+    const int64_t easy_end = (int64_t)ids.size();
+    append_ids(py::object(hard[q]).ptr(), n_candidates, ids);
+    a.hard_counts.push_back((int64_t)ids.size() - easy_end);
+    a.longest = std::max(a.longest, (int64_t)ids.size() - ptr.back());
+    ptr.push_back((int64_t)ids.size());
+    hard_ptr.push_back(hard_ptr.back() + a.hard_counts.back());
+  }
+  a.n = (int64_t)ids.size();
+  a.n_hard = hard_ptr.back();
+  if (a.n == 0) return a;
+  Tensor host = at::empty({2 * (Q + 1) + a.n}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
+  int64_t* h = (int64_t*)host.data_ptr();
+  h = std::copy(ptr.begin(), ptr.end(), h);
+  h = std::copy(hard_ptr.begin(), hard_ptr.end(), h);
+  std::copy(ids.begin(), ids.end(), h);
+  a.device = host.to(like.device(), /*non_blocking=*/true);
+  return a;
+}
+
+py::list split_ranks(const Tensor& ranks, const Answers& a) {
+  py::list out;
+  int64_t at = 0;
+  for (int64_t n : a.hard_counts) {
+    out.append(ranks.narrow(0, at, n));
+    at += n;
+  }
+  return out;
+}
+
+py::list filtered_ranks(Tensor logits, const py::sequence& easy, const py::sequence& hard) {
+  if (logits.dim() != 2 || logits.scalar_type() != at::kFloat || !logits.is_cuda())
+    throw py::type_error("logits must be a 2-D float32 CUDA tensor");
+  const int64_t Q = logits.size(0), N = logits.size(1);
+  c10::cuda::CUDAGuard guard(logits.device());
+  at::NoGradGuard no_grad;
+  logits = logits.contiguous();
+  const Answers a = pack_answers(easy, hard, Q, N, logits);
+  Tensor ranks = at::empty({a.n_hard}, logits.options().dtype(at::kLong));
+  if (a.n) {
+    Tensor ws = scratch(logits, smore_filtered_ranks_workspace_bytes(a.n));
+    Timed timed("filtered_ranks");
+    check(smore_hard_ranks(fptr(logits), Q, N, a.ptr(), a.ids(), a.n, a.longest, a.hard_ptr(), (int64_t*)ranks.data_ptr(),
+                           ws.data_ptr(), ws.numel(), stream_of(logits)),
+          "smore_hard_ranks");
+  }
+  return split_ranks(ranks, a);
+}
+
+py::list score_and_rank(int dist_id, const Tensor& table, const Tensor& first, const std::optional<Tensor>& second_opt,
+                        const py::sequence& easy, const py::sequence& hard, double gamma, double cen) {
+  if (table.scalar_type() != at::kFloat || !table.is_cuda() || !table.is_contiguous())
+    throw py::type_error("table must be a contiguous float32 CUDA tensor");
+  c10::cuda::CUDAGuard guard(table.device());
+  at::NoGradGuard no_grad;
+  const int64_t Q = first.size(0), N = table.size(0);
+  const Tensor q0 = first.reshape({Q, -1}).contiguous();
+  const Tensor q1 = second_opt ? second_opt->reshape({Q, -1}).contiguous() : Tensor();
+  const Answers a = pack_answers(easy, hard, Q, N, table);
+  Tensor ranks = at::empty({a.n_hard}, table.options().dtype(at::kLong));
+  if (a.n) {
+    Tensor ws = scratch(table, smore_score_filtered_ranks_workspace_bytes(Q, a.n));
+    Timed timed("score_filtered_ranks");
+    check(smore_score_hard_ranks(dist_id, fptr(table), N, fptr(q0), fptr(q1), Q, q0.size(1), gamma, cen, a.ptr(), a.ids(), a.n,
+                                 a.longest, a.hard_ptr(), (int64_t*)ranks.data_ptr(), ws.data_ptr(), ws.numel(),
+                                 stream_of(table)),
+          "smore_score_hard_ranks");
+  }
+  return split_ranks(ranks, a);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_host, mod) {
@@ -949,4 +1060,6 @@ PYBIND11_MODULE(_host, mod) {
   mod.def("rows_dist", &rows_dist);
   mod.def("dense_dist", &dense_dist);
   mod.def("path_embed", &path_embed);
+  mod.def("filtered_ranks", &filtered_ranks);
+  mod.def("score_and_rank", &score_and_rank);
 }

@@ -31,13 +31,16 @@ struct RankWorkspace {
 
 RankWorkspace carve_rank_workspace(void* workspace, size_t n_answers);
 
-// Per query: sort the answers best first (keys from logits[q, col], col = the answer's entity id, or
-// its position in answer_ids when cols_are_positions) and clear the histogram.
+// Per query: sort the answers best first and clear the histogram.  Keys come from logits[q, id of the
+// answer] ([n_queries, n_cols]), or, with per_answer, from logits[position in answer_ids].
 int rank_sort_answers(const float* logits, size_t n_cols, const int64_t* answer_ptr, const int64_t* answer_ids,
-                      bool cols_are_positions, size_t n_queries, size_t n_answers, size_t max_answers,
+                      bool per_answer, size_t n_queries, size_t n_answers, size_t max_answers,
                       const RankWorkspace& w, cudaStream_t st);
 
-// ranks[p] = candidates ahead of answer p - answers ahead of it + 1, in the caller's answer order
-int rank_finalize(const int64_t* answer_ptr, const RankWorkspace& w, int64_t* ranks, size_t n_queries, cudaStream_t st);
+// ranks[p] = candidates ahead of answer p - answers ahead of it + 1, in the caller's answer order.  With
+// hard_ptr ([n_queries + 1]) only the ranks of the hard answers are written - the last
+// hard_ptr[q + 1] - hard_ptr[q] of query q's list - sorted, from ranks[hard_ptr[q]] on.
+int rank_finalize(const int64_t* answer_ptr, const RankWorkspace& w, const int64_t* hard_ptr, size_t max_answers,
+                  int64_t* ranks, size_t n_queries, cudaStream_t st);
 
 }  // namespace smore

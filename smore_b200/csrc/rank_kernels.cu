@@ -33,7 +33,7 @@ constexpr size_t kRankMaxAnswers = 8192;   // per query: sorted in shared memory
 
 // one CTA per query; P = power of two >= the longest answer list
 __global__ void __launch_bounds__(kRankThreads)
-    rank_sort_answers_kernel(const float* __restrict__ logits, size_t n_candidates, int cols_are_positions,
+    rank_sort_answers_kernel(const float* __restrict__ logits, size_t n_candidates, int per_answer,
                              const int64_t* __restrict__ answer_ptr, const int64_t* __restrict__ answer_ids,
                              int P, uint32_t* __restrict__ sorted_logit, int64_t* __restrict__ sorted_id,
                              int32_t* __restrict__ perm) {
@@ -43,14 +43,14 @@ __global__ void __launch_bounds__(kRankThreads)
   const size_t q = blockIdx.x;
   const int64_t begin = answer_ptr[q];
   const int A = (int)(answer_ptr[q + 1] - begin);
-  const float* row = logits + q * n_candidates;
+  const float* row = logits + (per_answer ? 0 : q * n_candidates);
   for (int i = threadIdx.x; i < P; i += kRankThreads) {
     uint32_t k = 0;
     int32_t p = INT_MAX;
     if (i < A) {
       // the answer's logit sits in the column of its entity id, or (scores computed for the answers
-      // alone, one column per listed answer) in the column of its position in the list
-      const int64_t id = cols_are_positions ? begin + i : answer_ids[begin + i];
+      // alone, one per listed answer) at its position in the list
+      const int64_t id = per_answer ? begin + i : answer_ids[begin + i];
       k = (id >= 0 && (size_t)id < n_candidates) ? rank_key(row[id]) : 0u;
       p = i;
     }
@@ -140,34 +140,62 @@ __global__ void __launch_bounds__(kRankThreads)
     if (local[i]) atomicAdd(&hist[begin + i], local[i]);
 }
 
-// one CTA per query
+// one CTA per query; P = power of two >= the longest answer list (used with hard_ptr)
 __global__ void __launch_bounds__(kRankThreads)
     rank_finalize_kernel(const int64_t* __restrict__ answer_ptr, const int32_t* __restrict__ hist,
-                         const int32_t* __restrict__ perm, int64_t* __restrict__ ranks) {
+                         const int32_t* __restrict__ perm, const int64_t* __restrict__ hard_ptr, int P,
+                         int64_t* __restrict__ ranks) {
+  extern __shared__ unsigned char rank_smem[];
+  long long* vals = reinterpret_cast<long long*>(rank_smem);   // [P] ranks of the hard answers
   __shared__ long long seg[kRankThreads];
   const size_t q = blockIdx.x;
   const int64_t begin = answer_ptr[q];
   const int A = (int)(answer_ptr[q + 1] - begin);
+  const int n_hard = hard_ptr ? (int)(hard_ptr[q + 1] - hard_ptr[q]) : 0;
+  const int n_easy = A - n_hard;
   const int per = (A + kRankThreads - 1) / kRankThreads;
   const int i0 = threadIdx.x * per, i1 = min(A, i0 + per);
   long long s = 0;
   for (int i = i0; i < i1; ++i) s += hist[begin + i];
-  seg[threadIdx.x] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    long long run = 0;
-    for (int t = 0; t < kRankThreads; ++t) {
-      const long long v = seg[t];
-      seg[t] = run;
-      run += v;
-    }
+  // inclusive scan of the threads' sums: within warps, then over the warps
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  long long inc = s;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long t = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += t;
   }
+  if (lane == 31) seg[warp] = inc;
   __syncthreads();
-  long long ahead = seg[threadIdx.x];
+  long long ahead = inc - s;
+  for (int w = 0; w < warp; ++w) ahead += seg[w];
   for (int i = i0; i < i1; ++i) {
     ahead += hist[begin + i];                        // candidates (answers included) ahead of sorted answer i
-    ranks[begin + perm[begin + i]] = ahead - i + 1;  // i answers are ahead of it
+    const long long rank = ahead - i + 1;            // i answers are ahead of it
+    const int at = perm[begin + i];
+    if (hard_ptr == nullptr) ranks[begin + at] = rank;
+    else if (at >= n_easy) vals[at - n_easy] = rank;
   }
+  if (hard_ptr == nullptr) return;
+  int n = 1;
+  while (n < n_hard) n <<= 1;
+  for (int i = n_hard + threadIdx.x; i < n; i += kRankThreads) vals[i] = LLONG_MAX;
+  __syncthreads();
+  for (int size = 2; size <= n; size <<= 1)
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      for (int i = threadIdx.x; i < n; i += kRankThreads) {
+        const int j = i ^ stride;
+        if (j > i) {
+          const long long x = vals[i], y = vals[j];
+          if ((x > y) == ((i & size) == 0)) {
+            vals[i] = y;
+            vals[j] = x;
+          }
+        }
+      }
+      __syncthreads();
+    }
+  for (int i = threadIdx.x; i < n_hard; i += kRankThreads) ranks[hard_ptr[q] + i] = vals[i];
 }
 
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -188,7 +216,7 @@ RankWorkspace carve_rank_workspace(void* workspace, size_t n_answers) {
 }
 
 int rank_sort_answers(const float* logits, size_t n_cols, const int64_t* answer_ptr, const int64_t* answer_ids,
-                      bool cols_are_positions, size_t n_queries, size_t n_answers, size_t max_answers,
+                      bool per_answer, size_t n_queries, size_t n_answers, size_t max_answers,
                       const RankWorkspace& w, cudaStream_t st) {
   if (max_answers > kRankMaxAnswers)
     return fail(SMORE_ERR_TOO_LARGE, "filtered_ranks: at most %zu answers per query", kRankMaxAnswers);
@@ -199,12 +227,17 @@ int rank_sort_answers(const float* logits, size_t n_cols, const int64_t* answer_
   while ((size_t)P < max_answers) P <<= 1;
   if (int rc = allow_large_smem(rank_sort_answers_kernel, (int)(kRankMaxAnswers * 8), false)) return rc;
   rank_sort_answers_kernel<<<(unsigned)n_queries, kRankThreads, (size_t)P * 8, st>>>(
-      logits, n_cols, cols_are_positions ? 1 : 0, answer_ptr, answer_ids, P, w.sorted_logit, w.sorted_id, w.perm);
+      logits, n_cols, per_answer ? 1 : 0, answer_ptr, answer_ids, P, w.sorted_logit, w.sorted_id, w.perm);
   return check_launch("rank_sort_answers_kernel");
 }
 
-int rank_finalize(const int64_t* answer_ptr, const RankWorkspace& w, int64_t* ranks, size_t n_queries, cudaStream_t st) {
-  rank_finalize_kernel<<<(unsigned)n_queries, kRankThreads, 0, st>>>(answer_ptr, w.hist, w.perm, ranks);
+int rank_finalize(const int64_t* answer_ptr, const RankWorkspace& w, const int64_t* hard_ptr, size_t max_answers,
+                  int64_t* ranks, size_t n_queries, cudaStream_t st) {
+  int P = 1;
+  while ((size_t)P < max_answers) P <<= 1;
+  if (int rc = allow_large_smem(rank_finalize_kernel, (int)(kRankMaxAnswers * 8), false)) return rc;
+  rank_finalize_kernel<<<(unsigned)n_queries, kRankThreads, hard_ptr ? (size_t)P * 8 : 0, st>>>(answer_ptr, w.hist, w.perm,
+                                                                                              hard_ptr, P, ranks);
   return check_launch("rank_finalize_kernel");
 }
 
@@ -216,9 +249,9 @@ extern "C" {
 
 size_t smore_filtered_ranks_workspace_bytes(size_t n_answers) { return carve_rank_workspace(nullptr, n_answers).bytes; }
 
-int smore_filtered_ranks(const float* logits, size_t n_queries, size_t n_candidates, const int64_t* answer_ptr,
-                         const int64_t* answer_ids, size_t n_answers, size_t max_answers, int64_t* ranks,
-                         void* workspace, size_t workspace_bytes, void* stream) {
+static int filtered_ranks_impl(const float* logits, size_t n_queries, size_t n_candidates, const int64_t* answer_ptr,
+                               const int64_t* answer_ids, size_t n_answers, size_t max_answers, const int64_t* hard_ptr,
+                               int64_t* ranks, void* workspace, size_t workspace_bytes, void* stream) {
   if (n_queries == 0 || n_answers == 0) return SMORE_OK;
   if (!logits || !answer_ptr || !answer_ids || !ranks || !workspace)
     return fail(SMORE_ERR_NULL, "filtered_ranks: NULL pointer");
@@ -241,7 +274,22 @@ int smore_filtered_ranks(const float* logits, size_t n_queries, size_t n_candida
   rank_count_kernel<<<grid, kRankThreads, count_smem, st>>>(logits, n_candidates, answer_ptr, w.sorted_logit,
                                                             w.sorted_id, per_cta, w.hist);
   if (int rc = check_launch("rank_count_kernel")) return rc;
-  return rank_finalize(answer_ptr, w, ranks, n_queries, st);
+  return rank_finalize(answer_ptr, w, hard_ptr, max_answers, ranks, n_queries, st);
+}
+
+int smore_filtered_ranks(const float* logits, size_t n_queries, size_t n_candidates, const int64_t* answer_ptr,
+                         const int64_t* answer_ids, size_t n_answers, size_t max_answers, int64_t* ranks,
+                         void* workspace, size_t workspace_bytes, void* stream) {
+  return filtered_ranks_impl(logits, n_queries, n_candidates, answer_ptr, answer_ids, n_answers, max_answers, nullptr,
+                             ranks, workspace, workspace_bytes, stream);
+}
+
+int smore_hard_ranks(const float* logits, size_t n_queries, size_t n_candidates, const int64_t* answer_ptr,
+                     const int64_t* answer_ids, size_t n_answers, size_t max_answers, const int64_t* hard_ptr,
+                     int64_t* hard_ranks, void* workspace, size_t workspace_bytes, void* stream) {
+  if (!hard_ptr) return fail(SMORE_ERR_NULL, "hard_ranks: hard_ptr is NULL");
+  return filtered_ranks_impl(logits, n_queries, n_candidates, answer_ptr, answer_ids, n_answers, max_answers, hard_ptr,
+                             hard_ranks, workspace, workspace_bytes, stream);
 }
 
 }  // extern "C"

@@ -4,7 +4,7 @@
 //
 // Every (query, candidate) pair re-uses rows that other pairs also use, so this shape is bound by
 // fp32 ALU throughput and on-chip bandwidth, not by HBM: B*K*dim term evaluations against only
-// (B + K)*dim*4 bytes.  The forward kernel is tiled like a SIMT matrix product (a 64 x 64 tile of
+// (B + K)*dim*4 bytes.  The forward kernel is tiled like a SIMT matrix product (a 32 x 64 tile of
 // cells per CTA, operands staged through shared memory, 4 x 4 cells per thread); the backward
 // kernel evaluates every term once for both gradients: candidate-row gradients are summed in a fixed
 // order (registers, then across a thread-block cluster), query gradients by floating-point
@@ -23,10 +23,21 @@
 
 namespace smore {
 
-constexpr int kTileB = 64;     // queries per CTA tile
-constexpr int kTileK = 64;     // candidate rows per CTA tile
-constexpr int kTileD = 16;     // embedding dims staged per step
-constexpr int kTilePad = 4;    // keeps rows of the transposed tiles 16-byte aligned, off the same bank
+// One tile of scores: kTileB queries x kTileK candidate rows by kTileThreads threads, kCellsB x kCellsK
+// cells each.  32 queries per tile because that is what an evaluation batch and the ragged end of a
+// training batch have (64 left half the tile empty at 32 queries); a row of cells per thread re-uses
+// every operand four times from registers, which keeps shared-memory reads at 12 per 320 arithmetic
+// instructions (box distances).
+constexpr int kTileB = 32;
+constexpr int kTileK = 64;
+constexpr int kTileThreads = 128;
+constexpr int kCellsB = 4, kCellsK = 4;
+constexpr int kTileTx = kTileK / kCellsK;                 // thread columns: candidates tx + kTileTx * j
+constexpr int kTileTy = kTileThreads / kTileTx;           // thread rows: queries ty + kTileTy * i
+constexpr int kTileD = 32;                                // embedding dims staged per step
+constexpr int kTileStride = kTileD + 4;                   // floats per staged row: rows stay 16-byte aligned
+                                                          // and eight consecutive ones cover all 32 banks
+static_assert(kTileTy * kCellsB == kTileB && kTileTx * kCellsK == kTileK, "tile shape");
 
 struct SharedArgs {
   const float* ent;        // [K, W] or table when idx != nullptr
@@ -42,99 +53,132 @@ struct SharedArgs {
 // it.  (Defined here because this header is part of exactly one translation unit, dist_kernels.cu.)
 __device__ int g_async_status = 0;
 
-// Shared memory of one 64 x 64 tile of scores.
+// Shared memory of one tile: two stages of kTileD dims, filled by asynchronous copies while the other
+// one is being used.
+template <class Term>
+struct TileStage {
+  float q0[kTileB][kTileStride];
+  float q1[Term::kNQ == 2 ? kTileB : 1][kTileStride];
+  float e[Term::kMul][kTileK][kTileStride];
+};
 template <class Term>
 struct TileSmem {
-  float q0s[kTileD][kTileB + kTilePad];
-  float q1s[kTileD][kTileB + kTilePad];
-  float e0s[kTileD][kTileK + kTilePad];
-  float e1s[Term::kMul == 2 ? kTileD : 1][kTileK + kTilePad];
-  unsigned char ebad[kTileK];   // candidate rows of the tile whose id lay outside the table
+  TileStage<Term> stage[2];
+  long long rows[kTileK];       // table rows of the tile's candidates; -1: an id outside the table
 };
 
+__device__ __forceinline__ void copy16_async(void* smem, const void* gmem, bool ok) {
+  const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+  const int bytes = ok ? 16 : 0;   // 0: zero-fill, nothing is read
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(gmem), "r"(bytes) : "memory");
+}
+
 // Scores of the tile (queries b0.., candidates k0..) into acc: thread (ty, tx) owns queries
-// b0 + 4 ty + i and candidates k0 + 4 tx + j.  Every cell accumulates its terms in the order of the
-// embedding dim, one after the other, so a (query, candidate) pair gets the same value wherever it
-// falls in a tile and whatever the tile's neighbours are.
+// b0 + ty + kTileTy * i and candidates k0 + tx + kTileTx * j.  Every cell accumulates its terms in the
+// order of the embedding dim, one after the other, so a (query, candidate) pair gets the same value
+// wherever it falls in a tile and whatever the tile's neighbours are.  All threads of the CTA call this;
+// it starts with a barrier (the previous tile's shared memory is free again) and sets sm.rows.
+// (32 queries x 10.76M rows of dim 400, box distances: 57.3 ms with 64 x 64 tiles of half-empty query
+// rows, see kTileB.)
 template <class Term>
 __device__ __forceinline__ void tile_scores(const SharedArgs& a, TileSmem<Term>& sm, int b0, int k0,
-                                            float (&acc)[4][4][Term::kNOut]) {
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+                                            float (&acc)[kCellsB][kCellsK][Term::kNOut]) {
+  const int tx = threadIdx.x % kTileTx, ty = threadIdx.x / kTileTx;
   const int dim4 = a.dim >> 2;
   const size_t w4 = (size_t)dim4 * Term::kMul;
-  // staging role: one 16-byte piece of one row per operand per step
-  const int lrow = threadIdx.x >> 2, lq = threadIdx.x & 3;
-  const bool qrow_ok = b0 + lrow < a.B, erow_ok = k0 + lrow < a.K;
-  const float4* q0p = reinterpret_cast<const float4*>(a.first) + (size_t)(qrow_ok ? b0 + lrow : 0) * dim4;
-  const float4* q1p = reinterpret_cast<const float4*>(a.second) + (size_t)(qrow_ok ? b0 + lrow : 0) * dim4;
-  size_t erow = 0;
-  if (erow_ok) {
-    const long long r = a.idx ? checked_row_id(a.idx, k0 + lrow, a.n_rows, &g_async_status) : (long long)(k0 + lrow);
-    erow = r < 0 ? 0 : (size_t)r;
-    if (lq == 0) sm.ebad[lrow] = r < 0;
-  } else if (lq == 0) {
-    sm.ebad[lrow] = 0;
+  __syncthreads();
+  if (threadIdx.x < kTileK) {
+    const int k = k0 + threadIdx.x;
+    sm.rows[threadIdx.x] = k >= a.K ? 0 : a.idx ? checked_row_id(a.idx, k, a.n_rows, &g_async_status) : (long long)k;
   }
-  const float4* e0p = reinterpret_cast<const float4*>(a.ent) + erow * w4;
+  __syncthreads();
+  // staging role: the 16-byte pieces lc of rows lr, lr + 16, ... of every operand
+  constexpr int kPieces = kTileD / 4, kRowsPerPass = kTileThreads / kPieces;
+  const int lc = threadIdx.x % kPieces, lr = threadIdx.x / kPieces;
+  const float4* ent4 = reinterpret_cast<const float4*>(a.ent);
+  const float4* first4 = reinterpret_cast<const float4*>(a.first);
+  const float4* second4 = reinterpret_cast<const float4*>(a.second);
+  auto stage = [&](int which, int d0) {
+    TileStage<Term>& st = sm.stage[which];
+    const int d4 = (d0 >> 2) + lc;
+    const bool d_ok = d4 < dim4;
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+    for (int r = lr; r < kTileB; r += kRowsPerPass) {
+      const bool ok = d_ok && b0 + r < a.B;
+      const size_t at = ok ? (size_t)(b0 + r) * dim4 + d4 : 0;
+      copy16_async(&st.q0[r][lc * 4], first4 + at, ok);
+      if (Term::kNQ == 2) copy16_async(&st.q1[r][lc * 4], second4 + at, ok);
+    }
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int r = lr; r < kTileK; r += kRowsPerPass) {
+      const bool ok = d_ok && k0 + r < a.K;
+      const size_t at = ok ? (size_t)max(sm.rows[r], 0LL) * w4 + d4 : 0;
+      copy16_async(&st.e[0][r][lc * 4], ent4 + at, ok);
+      if (Term::kMul == 2) copy16_async(&st.e[Term::kMul - 1][r][lc * 4], ent4 + (ok ? at + dim4 : 0), ok);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int i = 0; i < kCellsB; ++i)
+#pragma unroll
+    for (int j = 0; j < kCellsK; ++j)
 #pragma unroll
       for (int o = 0; o < Term::kNOut; ++o) acc[i][j][o] = 0.f;
 
-  const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int d0 = 0; d0 < a.dim; d0 += kTileD) {
-    const int d4 = (d0 >> 2) + lq;
-    const bool d_ok = d4 < dim4;
-    const float4 vq0 = (qrow_ok && d_ok) ? __ldg(q0p + d4) : z4;
-    const float4 vq1 = (Term::kNQ == 2 && qrow_ok && d_ok) ? __ldg(q1p + d4) : z4;
-    const float4 ve0 = (erow_ok && d_ok) ? __ldg(e0p + d4) : z4;
-    const float4 ve1 = (Term::kMul == 2 && erow_ok && d_ok) ? __ldg(e0p + dim4 + d4) : z4;
-    __syncthreads();  // the previous step's tiles are no longer being read
-    sm.q0s[lq * 4 + 0][lrow] = vq0.x; sm.q0s[lq * 4 + 1][lrow] = vq0.y; sm.q0s[lq * 4 + 2][lrow] = vq0.z; sm.q0s[lq * 4 + 3][lrow] = vq0.w;
-    if (Term::kNQ == 2) {
-      sm.q1s[lq * 4 + 0][lrow] = vq1.x; sm.q1s[lq * 4 + 1][lrow] = vq1.y; sm.q1s[lq * 4 + 2][lrow] = vq1.z; sm.q1s[lq * 4 + 3][lrow] = vq1.w;
-    }
-    sm.e0s[lq * 4 + 0][lrow] = ve0.x; sm.e0s[lq * 4 + 1][lrow] = ve0.y; sm.e0s[lq * 4 + 2][lrow] = ve0.z; sm.e0s[lq * 4 + 3][lrow] = ve0.w;
-    if (Term::kMul == 2) {
-      sm.e1s[lq * 4 + 0][lrow] = ve1.x; sm.e1s[lq * 4 + 1][lrow] = ve1.y; sm.e1s[lq * 4 + 2][lrow] = ve1.z; sm.e1s[lq * 4 + 3][lrow] = ve1.w;
-    }
-    __syncthreads();
-    const int dcount = min(kTileD, a.dim - d0);
-#pragma unroll 4
-    for (int dd = 0; dd < dcount; ++dd) {
-      const float4 q0 = *reinterpret_cast<const float4*>(&sm.q0s[dd][ty * 4]);
-      const float4 q1 = Term::kNQ == 2 ? *reinterpret_cast<const float4*>(&sm.q1s[dd][ty * 4]) : q0;
-      const float4 e0 = *reinterpret_cast<const float4*>(&sm.e0s[dd][tx * 4]);
-      const float4 e1 = Term::kMul == 2 ? *reinterpret_cast<const float4*>(&sm.e1s[dd][tx * 4]) : e0;
-      const float qa[4] = {q0.x, q0.y, q0.z, q0.w}, qb[4] = {q1.x, q1.y, q1.z, q1.w};
-      const float ea[4] = {e0.x, e0.y, e0.z, e0.w}, eb[4] = {e1.x, e1.y, e1.z, e1.w};
+  stage(0, 0);
+  int cur = 0;
+  for (int d0 = 0; d0 < a.dim; d0 += kTileD, cur ^= 1) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();   // this stage has landed for everyone, and nobody reads the other one any more
+    if (d0 + kTileD < a.dim) stage(cur ^ 1, d0 + kTileD);
+    const TileStage<Term>& st = sm.stage[cur];
+    const int pieces = min(kPieces, dim4 - (d0 >> 2));
+#pragma unroll 1
+    for (int p = 0; p < pieces; ++p) {
+      float4 q0[kCellsB], q1[kCellsB], e0[kCellsK], e1[kCellsK];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < kCellsB; ++i) {
+        q0[i] = *reinterpret_cast<const float4*>(&st.q0[ty + kTileTy * i][p * 4]);
+        q1[i] = Term::kNQ == 2 ? *reinterpret_cast<const float4*>(&st.q1[ty + kTileTy * i][p * 4]) : q0[i];
+      }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) Term::fwd(ea[j], eb[j], qa[i], qb[i], acc[i][j]);
+      for (int j = 0; j < kCellsK; ++j) {
+        e0[j] = *reinterpret_cast<const float4*>(&st.e[0][tx + kTileTx * j][p * 4]);
+        e1[j] = Term::kMul == 2 ? *reinterpret_cast<const float4*>(&st.e[Term::kMul - 1][tx + kTileTx * j][p * 4]) : e0[j];
+      }
+#pragma unroll
+      for (int i = 0; i < kCellsB; ++i)
+#pragma unroll
+        for (int j = 0; j < kCellsK; ++j) {
+          Term::fwd(e0[j].x, e1[j].x, q0[i].x, q1[i].x, acc[i][j]);
+          Term::fwd(e0[j].y, e1[j].y, q0[i].y, q1[i].y, acc[i][j]);
+          Term::fwd(e0[j].z, e1[j].z, q0[i].z, q1[i].z, acc[i][j]);
+          Term::fwd(e0[j].w, e1[j].w, q0[i].w, q1[i].w, acc[i][j]);
+        }
     }
   }
 }
 
+// Grid: one CTA per tile, query tiles of the same candidates next to each other (they share the rows in L2).
 template <class Term>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kTileThreads)
     shared_forward_kernel(SharedArgs a, float* __restrict__ dst0, float* __restrict__ dst1) {
-  __shared__ __align__(16) TileSmem<Term> sm;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int b0 = blockIdx.y * kTileB, k0 = blockIdx.x * kTileK;
-  float acc[4][4][Term::kNOut];
+  extern __shared__ __align__(16) unsigned char tile_smem[];
+  TileSmem<Term>& sm = *reinterpret_cast<TileSmem<Term>*>(tile_smem);
+  const int tx = threadIdx.x % kTileTx, ty = threadIdx.x / kTileTx;
+  const int q_tiles = (a.B + kTileB - 1) / kTileB;
+  const int b0 = (int)(blockIdx.x % q_tiles) * kTileB, k0 = (int)(blockIdx.x / q_tiles) * kTileK;
+  float acc[kCellsB][kCellsK][Term::kNOut];
   tile_scores<Term>(a, sm, b0, k0, acc);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int b = b0 + ty * 4 + i;
+  for (int i = 0; i < kCellsB; ++i) {
+    const int b = b0 + ty + kTileTy * i;
     if (b >= a.B) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int k = k0 + tx * 4 + j;
+    for (int j = 0; j < kCellsK; ++j) {
+      const int k = k0 + tx + kTileTx * j;
       if (k < a.K) {
-        const bool bad = sm.ebad[tx * 4 + j];   // written before the first barrier of the tile loop
+        const bool bad = sm.rows[tx + kTileTx * j] < 0;
         dst0[(size_t)b * a.K + k] = bad ? NAN : acc[i][j][0];
         if (Term::kNOut == 2) dst1[(size_t)b * a.K + k] = bad ? NAN : acc[i][j][Term::kNOut - 1];
       }

@@ -6,7 +6,7 @@ a query against every entity (smore/training/train_process.py:113-153).
     logs  = ranking_metrics(ranks)                      # MRR, HITS1/3/10, HITS1max per query
 
 `filtered_ranks` replaces argsort + scatter over the N logits by a count per answer
-(smore_filtered_ranks in libsmore_b200.so); there is no CPU path.
+(smore_hard_ranks in libsmore_b200.so); there is no CPU path.
 """
 import torch
 
@@ -22,54 +22,7 @@ def filtered_ranks(logits, easy_answers, hard_answers):
     Returns a list of Q int64 CUDA tensors: the ranks of each query's hard answers in ascending
     order, the quantity `cur_ranking[masks]` of train_process.py:140-141.
     """
-    if logits.dim() != 2 or logits.dtype != torch.float32 or not logits.is_cuda:
-        raise TypeError("logits must be a 2-D float32 CUDA tensor")
-    logits = logits.contiguous()
-    Q, N = logits.shape
-    if len(easy_answers) != Q or len(hard_answers) != Q:
-        raise ValueError("one easy and one hard answer list per query")
-    ptr, ids, hard_mask = [0], [], []
-    for easy, hard in zip(easy_answers, hard_answers):
-        easy, hard = list(easy), list(hard)
-        ids.extend(easy)
-        ids.extend(hard)
-        hard_mask.extend([False] * len(easy) + [True] * len(hard))
-        ptr.append(len(ids))
-    n_answers = len(ids)
-    if n_answers == 0:
-        return [torch.empty(0, dtype=torch.int64, device=logits.device) for _ in range(Q)]
-    if any((i < 0 or i >= N) for i in ids):
-        raise ValueError("answer ids must lie in [0, %d)" % N)
-    max_answers = max(b - a for a, b in zip(ptr[:-1], ptr[1:]))
-    dev = logits.device
-    d_ptr = torch.tensor(ptr, dtype=torch.int64, device=dev)
-    d_ids = torch.tensor(ids, dtype=torch.int64, device=dev)
-    ranks = torch.empty(n_answers, dtype=torch.int64, device=dev)
-    L = _lib.lib()
-    ws = torch.empty(L.smore_filtered_ranks_workspace_bytes(n_answers), dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev), _lib.timed("filtered_ranks"):
-        _lib.check(L.smore_filtered_ranks(logits.data_ptr(), Q, N, d_ptr.data_ptr(), d_ids.data_ptr(), n_answers,
-                                          max_answers, ranks.data_ptr(), ws.data_ptr(), ws.numel(),
-                                          torch.cuda.current_stream(dev).cuda_stream), "smore_filtered_ranks")
-    mask = torch.tensor(hard_mask, dtype=torch.bool, device=dev)
-    out = []
-    for q in range(Q):
-        r = ranks[ptr[q]:ptr[q + 1]][mask[ptr[q]:ptr[q + 1]]]
-        out.append(torch.sort(r)[0])
-    return out
-
-
-def _answer_lists(easy_answers, hard_answers, n_candidates):
-    ptr, ids, hard_mask = [0], [], []
-    for easy, hard in zip(easy_answers, hard_answers):
-        easy, hard = list(easy), list(hard)
-        ids.extend(easy)
-        ids.extend(hard)
-        hard_mask.extend([False] * len(easy) + [True] * len(hard))
-        ptr.append(len(ids))
-    if any((i < 0 or i >= n_candidates) for i in ids):
-        raise ValueError("answer ids must lie in [0, %d)" % n_candidates)
-    return ptr, ids, hard_mask
+    return _lib.host().filtered_ranks(logits, easy_answers, hard_answers)
 
 
 _SCORE_IDS = {"box": _lib.BOX_BOTH_ID, "vec": _lib.DIST_IDS["l1"], "l1": _lib.DIST_IDS["l1"], "l2": _lib.DIST_IDS["l2"],
@@ -80,7 +33,7 @@ _SCORE_IDS = {"box": _lib.BOX_BOTH_ID, "vec": _lib.DIST_IDS["l1"], "l1": _lib.DI
 def score_and_rank(geo, table, query, easy_answers, hard_answers, gamma=0.0, cen=0.0):
     """The evaluation step in one call: score Q queries against every row of `table` with the model's
     logit and return the filtered ranks of their hard answers, without materialising the [Q, N]
-    logits (smore_score_filtered_ranks).
+    logits (smore_score_hard_ranks).
 
     geo      "box" (gamma - d_out - cen * d_in), "vec" / "l1" / "rotate" (gamma - d), "l2" (gamma - sqrt(d)),
              "complex" / "distmult" (the similarity)
@@ -89,32 +42,8 @@ def score_and_rank(geo, table, query, easy_answers, hard_answers, gamma=0.0, cen
     Returns what filtered_ranks returns for the logits the distance ops would have produced."""
     if geo not in _SCORE_IDS:
         raise ValueError("geo must be one of %s" % sorted(_SCORE_IDS))
-    parts = [q.reshape(q.shape[0], -1).contiguous() for q in query]
-    Q, dim = parts[0].shape
-    N = table.shape[0]
-    if table.dtype != torch.float32 or not table.is_cuda or not table.is_contiguous():
-        raise TypeError("table must be a contiguous float32 CUDA tensor")
-    ptr, ids, hard_mask = _answer_lists(easy_answers, hard_answers, N)
-    if len(ptr) != Q + 1:
-        raise ValueError("one easy and one hard answer list per query")
-    n_answers = len(ids)
-    dev = table.device
-    if n_answers == 0:
-        return [torch.empty(0, dtype=torch.int64, device=dev) for _ in range(Q)]
-    max_answers = max(b - a for a, b in zip(ptr[:-1], ptr[1:]))
-    d_ptr = torch.tensor(ptr, dtype=torch.int64, device=dev)
-    d_ids = torch.tensor(ids, dtype=torch.int64, device=dev)
-    ranks = torch.empty(n_answers, dtype=torch.int64, device=dev)
-    L = _lib.lib()
-    ws = torch.empty(L.smore_score_filtered_ranks_workspace_bytes(Q, n_answers), dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev), _lib.timed("score_filtered_ranks"):
-        _lib.check(L.smore_score_filtered_ranks(
-            _SCORE_IDS[geo], table.data_ptr(), N, parts[0].data_ptr(), parts[1].data_ptr() if len(parts) > 1 else None,
-            Q, dim, float(gamma), float(cen), d_ptr.data_ptr(), d_ids.data_ptr(), n_answers, max_answers,
-            ranks.data_ptr(), ws.data_ptr(), ws.numel(), torch.cuda.current_stream(dev).cuda_stream),
-            "smore_score_filtered_ranks")
-    mask = torch.tensor(hard_mask, dtype=torch.bool, device=dev)
-    return [torch.sort(ranks[ptr[q]:ptr[q + 1]][mask[ptr[q]:ptr[q + 1]]])[0] for q in range(Q)]
+    return _lib.host().score_and_rank(_SCORE_IDS[geo], table, query[0], query[1] if len(query) > 1 else None, easy_answers,
+                                      hard_answers, float(gamma), float(cen))
 
 
 def ranking_metrics(hard_ranks):
