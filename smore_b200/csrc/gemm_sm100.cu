@@ -141,6 +141,14 @@ static int run_precision(int precision, const float* A, const float* B, float* D
     return fail(SMORE_ERR_BAD_DIST, "unknown dot precision %d", precision);
   const bool fast = precision == SMORE_DOT_FP32;
   int code;
+  // Building the tensor maps is a driver call and needs a current context; a thread whose first CUDA call
+  // this is (autograd's) has none until it sets its device.
+  static thread_local int bound = -1;
+  int dev = 0;
+  if (!need && cudaGetDevice(&dev) == cudaSuccess && dev != bound) {
+    if (cudaSetDevice(dev) != cudaSuccess) return fail(SMORE_ERR_CUDA, "dot: cudaSetDevice failed");
+    bound = dev;
+  }
   TwoSmRun wide = M >= 256 ? two_sm() : nullptr;
   if (wide != nullptr) {
     code = wide(kLayout, fast ? 1 : 0, A, B, D, M, N, K, ws, ws_bytes, st, need);
