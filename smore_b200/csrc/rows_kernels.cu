@@ -58,15 +58,28 @@ __global__ void __launch_bounds__(256)
 constexpr int kScanThreads = 256;
 constexpr int kWordsPerThread = 4;
 constexpr int kWordsPerBlock = kScanThreads * kWordsPerThread;  // 1024 words = 32768 ids
+constexpr int kIdLists = 8;                                     // id lists of one call
+
+// The ids of a call: up to kIdLists lists, one after the other.
+struct IdLists {
+  const int64_t* ptr[kIdLists];
+  size_t end[kIdLists];     // position of the first id after list i
+  __device__ __forceinline__ int64_t at(size_t p) const {
+    int i = 0;
+    while (i < kIdLists - 1 && p >= end[i]) ++i;
+    return ptr[i][i == 0 ? p : p - end[i - 1]];
+  }
+};
 
 struct UniqueWorkspace {
   uint32_t* bitmap;      // [nwords]   bit v set <=> id v occurs
-  uint32_t* wordprefix;  // [nwords]   distinct ids below word w
-  uint32_t* blocksum;    // [nblocks]  distinct ids per 1024-word block, then their exclusive scan
+  uint32_t* done;        // blocks of the prefix kernel that have finished (directly behind the bitmap)
+  uint32_t* wordprefix;  // [nwords]   distinct ids below word w within its 1024-word block
+  uint32_t* blocksum;    // [nblocks]  distinct ids per block, then their exclusive scan
   size_t nwords, nblocks, bytes;
 };
 
-static size_t round256(size_t x) { return (x + 255) & ~(size_t)255; }
+static constexpr size_t round256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 static UniqueWorkspace carve_unique_workspace(void* base, size_t n_table_rows) {
   UniqueWorkspace w;
@@ -76,147 +89,151 @@ static UniqueWorkspace carve_unique_workspace(void* base, size_t n_table_rows) {
   const size_t b2 = round256(w.nblocks * sizeof(uint32_t));
   char* p = static_cast<char*>(base);
   w.bitmap = reinterpret_cast<uint32_t*>(p);
-  w.wordprefix = reinterpret_cast<uint32_t*>(p + b0);
-  w.blocksum = reinterpret_cast<uint32_t*>(p + 2 * b0);
-  w.bytes = 2 * b0 + b2;
+  w.done = reinterpret_cast<uint32_t*>(p + w.nwords * sizeof(uint32_t));
+  w.wordprefix = reinterpret_cast<uint32_t*>(p + b0 + 256);
+  w.blocksum = reinterpret_cast<uint32_t*>(p + 2 * b0 + 256);
+  w.bytes = 2 * b0 + 256 + b2;
   return w;
 }
 
+// Marks the ids' bits and clears the multiplicities.  Small tables: a CTA collects its bits in shared
+// memory first (few words, each set by many ids: 66k ids over 14,505 rows took 11 us of serialised atomics
+// on 454 words).
+constexpr size_t kLocalWords = 8192;   // tables of up to 262,144 rows
+template <bool LOCAL>
 __global__ void __launch_bounds__(256)
-    unique_mark_kernel(const int64_t* __restrict__ idx, size_t n, const int32_t* __restrict__ n_dev,
-                       size_t n_table_rows, uint32_t* __restrict__ bitmap, int32_t* __restrict__ n_unique) {
+    unique_mark_kernel(IdLists ids, size_t n, const int32_t* __restrict__ n_dev, size_t n_table_rows, size_t nwords,
+                       uint32_t* __restrict__ bitmap, int32_t* __restrict__ counts) {
+  extern __shared__ uint32_t local_bits[];   // [nwords] when LOCAL
+  if (LOCAL) {
+    for (size_t w = threadIdx.x; w < nwords; w += blockDim.x) local_bits[w] = 0;
+    __syncthreads();
+  }
+  const size_t stride = (size_t)gridDim.x * blockDim.x, p0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (size_t p = p0; p < n; p += stride) counts[p] = 0;
   if (n_dev != nullptr) n = min(n, (size_t)max(n_dev[0], 0));   // the caller's count lives on the device
-  for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < n;
-       p += (size_t)gridDim.x * blockDim.x) {
-    const int64_t v = idx[p];
+  for (size_t p = p0; p < n; p += stride) {
+    const int64_t v = ids.at(p);
     if (v >= 0 && (size_t)v < n_table_rows) {
       const uint32_t bit = 1u << (v & 31);
-      uint32_t* w = bitmap + (v >> 5);
+      uint32_t* w = (LOCAL ? local_bits : bitmap) + (v >> 5);
       if (!(*w & bit)) atomicOr(w, bit);
-    } else {
-      atomicAdd(n_unique + 1, 1);
+    }
+  }
+  if (LOCAL) {
+    __syncthreads();
+    for (size_t w = threadIdx.x; w < nwords; w += blockDim.x) {
+      const uint32_t bits = local_bits[w];
+      if (bits & ~bitmap[w]) atomicOr(bitmap + w, bits);
     }
   }
 }
 
-__device__ __forceinline__ uint32_t block_sum_256(uint32_t v, uint32_t* sh) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int m = 16; m > 0; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
-  if (lane == 0) sh[warp] = v;
-  __syncthreads();
-  uint32_t t = 0;
-#pragma unroll
-  for (int w = 0; w < kScanThreads / 32; ++w) t += sh[w];
-  __syncthreads();
-  return t;
-}
-
+// Distinct ids below every word within its block of 1024 words; the block that finishes last turns the
+// blocks' sums into their exclusive scan.  n_unique = {distinct ids, 0}.
 __global__ void __launch_bounds__(kScanThreads)
-    unique_blocksum_kernel(const uint32_t* __restrict__ bitmap, size_t nwords,
-                           uint32_t* __restrict__ blocksum) {
-  __shared__ uint32_t sh[kScanThreads / 32];
-  const size_t w0 = (size_t)blockIdx.x * kWordsPerBlock + (size_t)threadIdx.x * kWordsPerThread;
-  uint32_t c = 0;
-#pragma unroll
-  for (int k = 0; k < kWordsPerThread; ++k)
-    if (w0 + k < nwords) c += __popc(bitmap[w0 + k]);
-  const uint32_t t = block_sum_256(c, sh);
-  if (threadIdx.x == 0) blocksum[blockIdx.x] = t;
-}
-
-// exclusive scan of blocksum in place by one CTA; total -> n_unique[0]
-__global__ void __launch_bounds__(1024)
-    unique_scan_blocks_kernel(uint32_t* __restrict__ blocksum, size_t nblocks,
-                              int32_t* __restrict__ n_unique) {
-  __shared__ uint32_t warp_tot[32];
-  __shared__ uint32_t carry_sh;
+    unique_prefix_kernel(const uint32_t* __restrict__ bitmap, size_t nwords, uint32_t* __restrict__ wordprefix,
+                         uint32_t* blocksum, size_t nblocks, uint32_t* done, int32_t* __restrict__ n_unique) {
+  __shared__ uint32_t warp_tot[kScanThreads / 32];
+  __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) carry_sh = 0;
-  __syncthreads();
-  for (size_t base = 0; base < nblocks; base += 1024) {
-    const size_t i = base + threadIdx.x;
-    const uint32_t v = i < nblocks ? blocksum[i] : 0;
+  // inclusive scan over the CTA of one value per thread; every thread gets the total too
+  auto scan = [&](uint32_t v, uint32_t* total) {
     uint32_t inc = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
       if (lane >= o) inc += t;
     }
+    __syncthreads();
     if (lane == 31) warp_tot[warp] = inc;
     __syncthreads();
-    if (warp == 0) {
-      uint32_t w = warp_tot[lane];
+    uint32_t before = 0, all = 0;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, w, o);
-        if (lane >= o) w += t;
-      }
-      warp_tot[lane] = w;  // inclusive over warps
+    for (int w = 0; w < kScanThreads / 32; ++w) {
+      if (w < warp) before += warp_tot[w];
+      all += warp_tot[w];
     }
-    __syncthreads();
-    const uint32_t carry = carry_sh;
-    const uint32_t before_warp = warp ? warp_tot[warp - 1] : 0;
-    if (i < nblocks) blocksum[i] = carry + before_warp + inc - v;
-    __syncthreads();
-    if (threadIdx.x == 0) carry_sh = carry + warp_tot[31];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) n_unique[0] = (int32_t)carry_sh;
-}
-
-__global__ void __launch_bounds__(kScanThreads)
-    unique_wordprefix_kernel(const uint32_t* __restrict__ bitmap, size_t nwords,
-                             const uint32_t* __restrict__ blockoff, uint32_t* __restrict__ wordprefix) {
-  __shared__ uint32_t warp_tot[kScanThreads / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    *total = all;
+    return before + inc;
+  };
   const size_t w0 = (size_t)blockIdx.x * kWordsPerBlock + (size_t)threadIdx.x * kWordsPerThread;
   uint32_t c[kWordsPerThread];
-  uint32_t mine = 0;
+  uint32_t mine = 0, total;
 #pragma unroll
   for (int k = 0; k < kWordsPerThread; ++k) {
     c[k] = (w0 + k < nwords) ? __popc(bitmap[w0 + k]) : 0;
     mine += c[k];
   }
-  uint32_t inc = mine;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += t;
-  }
-  if (lane == 31) warp_tot[warp] = inc;
-  __syncthreads();
-  uint32_t before = blockoff[blockIdx.x];
-  for (int w = 0; w < warp; ++w) before += warp_tot[w];
-  uint32_t run = before + inc - mine;
+  uint32_t run = scan(mine, &total) - mine;
 #pragma unroll
   for (int k = 0; k < kWordsPerThread; ++k) {
     if (w0 + k < nwords) wordprefix[w0 + k] = run;
     run += c[k];
   }
-}
-
-__global__ void __launch_bounds__(256)
-    unique_assign_kernel(const int64_t* __restrict__ idx, size_t n, const int32_t* __restrict__ n_dev,
-                         size_t n_table_rows, const uint32_t* __restrict__ bitmap,
-                         const uint32_t* __restrict__ wordprefix, int64_t* __restrict__ uniq,
-                         int32_t* __restrict__ inverse, int32_t* __restrict__ counts) {
-  if (n_dev != nullptr) n = min(n, (size_t)max(n_dev[0], 0));
-  for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < n;
-       p += (size_t)gridDim.x * blockDim.x) {
-    const int64_t v = idx[p];
-    if (v < 0 || (size_t)v >= n_table_rows) {
-      inverse[p] = -1;
-      continue;
-    }
-    const uint32_t word = bitmap[v >> 5];
-    const uint32_t below = word & ((1u << (v & 31)) - 1u);
-    const int32_t s = (int32_t)(wordprefix[v >> 5] + __popc(below));
-    inverse[p] = s;
-    if (atomicAdd(counts + s, 1) == 0) uniq[s] = v;
+  if (threadIdx.x == 0) {
+    blocksum[blockIdx.x] = total;
+    __threadfence();
+    last = atomicAdd(done, 1u) == (uint32_t)(nblocks - 1);
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  uint32_t carry = 0;
+  for (size_t base = 0; base < nblocks; base += kScanThreads) {
+    const size_t i = base + threadIdx.x;
+    const uint32_t v = i < nblocks ? __ldcg(blocksum + i) : 0;
+    const uint32_t inc = scan(v, &total);
+    if (i < nblocks) blocksum[i] = carry + inc - v;
+    carry += total;
+  }
+  if (threadIdx.x == 0) {
+    n_unique[0] = (int32_t)carry;
+    n_unique[1] = 0;
   }
 }
 
+// Inverse map, multiplicities and the sorted list; with g_rows the gradient rows that more than one position
+// contributes to are cleared (by the warp of the second position of each).
+__global__ void __launch_bounds__(256)
+    unique_assign_kernel(IdLists ids, size_t n, const int32_t* __restrict__ n_dev, size_t n_table_rows,
+                         const uint32_t* __restrict__ bitmap, const uint32_t* __restrict__ wordprefix,
+                         const uint32_t* __restrict__ blockoff, int64_t* __restrict__ uniq,
+                         int32_t* __restrict__ inverse, int32_t* __restrict__ counts, int32_t* __restrict__ n_unique,
+                         float* __restrict__ g_rows, size_t width) {
+  if (n_dev != nullptr) n = min(n, (size_t)max(n_dev[0], 0));
+  const int lane = threadIdx.x & 31;
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  for (size_t first = (size_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); first < n; first += stride) {
+    const size_t p = first + lane;
+    int32_t s = -1, before = 0;
+    if (p < n) {
+      const int64_t v = ids.at(p);
+      if (v < 0 || (size_t)v >= n_table_rows) {
+        atomicAdd(n_unique + 1, 1);
+      } else {
+        const uint32_t word = bitmap[v >> 5];
+        const uint32_t below = word & ((1u << (v & 31)) - 1u);
+        s = (int32_t)(blockoff[(v >> 5) / kWordsPerBlock] + wordprefix[v >> 5] + __popc(below));
+        before = atomicAdd(counts + s, 1);
+        if (before == 0) uniq[s] = v;
+      }
+      inverse[p] = s;
+    }
+    if (g_rows == nullptr) continue;
+    unsigned todo = __ballot_sync(0xffffffffu, s >= 0 && before == 1);
+    while (todo) {
+      const int l = __ffs(todo) - 1;
+      todo &= todo - 1;
+      float* r = g_rows + (size_t)__shfl_sync(0xffffffffu, s, l) * width;
+      if ((width & 3) == 0) {
+        for (size_t d = lane; d < (width >> 2); d += kWarp) reinterpret_cast<float4*>(r)[d] = make_float4(0.f, 0.f, 0.f, 0.f);
+      } else {
+        for (size_t d = lane; d < width; d += kWarp) r[d] = 0.f;
+      }
+    }
+  }
+}
 
 // ----------------------------------------------------------------------------------------
 // sorted unique of a SHORT id list (a step's anchor lookups: about a thousand ids) over a LARGE id
@@ -231,7 +248,7 @@ constexpr int kSmallPosBits = 12;          // position within the call, packed b
 constexpr unsigned long long kSmallInvalid = ~0ull;
 
 __global__ void __launch_bounds__(kSmallUniqueThreads)
-    unique_small_kernel(const int64_t* __restrict__ idx, int n, size_t n_table_rows, int P,
+    unique_small_kernel(IdLists ids, int n, size_t n_table_rows, int P,
                         int64_t* __restrict__ uniq, int32_t* __restrict__ inverse, int32_t* __restrict__ counts,
                         int32_t* __restrict__ n_unique) {
   extern __shared__ unsigned long long keys[];   // [P], P = power of two >= n
@@ -244,7 +261,7 @@ __global__ void __launch_bounds__(kSmallUniqueThreads)
   for (int i = tid; i < P; i += kSmallUniqueThreads) {
     unsigned long long k = kSmallInvalid;
     if (i < n) {
-      const int64_t v = idx[i];
+      const int64_t v = ids.at(i);
       if (v >= 0 && (size_t)v < n_table_rows) k = ((unsigned long long)v << kSmallPosBits) | (unsigned)i;
       else ++bad;
       counts[i] = 0;
@@ -310,7 +327,7 @@ __global__ void __launch_bounds__(kSmallUniqueThreads)
   }
   // positions whose id was out of range
   for (int i = tid; i < n; i += kSmallUniqueThreads) {
-    const int64_t v = idx[i];
+    const int64_t v = ids.at(i);
     if (v < 0 || (size_t)v >= n_table_rows) inverse[i] = -1;
   }
   if (tid == 0) {
@@ -423,7 +440,8 @@ __global__ void __launch_bounds__(256) adam_rows_reg_kernel(UpdateArgs a) {
           if (!ROWWISE) v[j] = v4[d];
         }
       }
-      float denom = 0.f, v_old = 0.f, v_new = 0.f;
+      RowDenom denom = {1.f, 1.f};
+      float v_old = 0.f, v_new = 0.f;
       if (ROWWISE) {
         v_old = a.v[row];
         float s = 0.f;
@@ -432,7 +450,7 @@ __global__ void __launch_bounds__(256) adam_rows_reg_kernel(UpdateArgs a) {
           if (lane + 32 * j < w4) s += g[j].x * g[j].x + g[j].y * g[j].y + g[j].z * g[j].z + g[j].w * g[j].w;
         const float g2mean = warp_sum(s) / (float)a.width;
         v_new = v_old * a.beta2 + g2mean * a.omb2;
-        denom = sqrtf(v_new) / a.sqrt_bc2 + a.eps;
+        denom = rowwise_denom(v_new, a);
       }
 #pragma unroll
       for (int j = 0; j < NCH; ++j) {
@@ -533,7 +551,7 @@ __global__ void __launch_bounds__(256) sparse_update_rows_kernel(UpdateArgs a) {
       if (a.squeeze) {
         const float v_old = a.v[row];
         const float v_new = v_old * a.beta2 + g2mean * a.omb2;
-        const float denom = sqrtf(v_new) / a.sqrt_bc2 + a.eps;
+        const RowDenom denom = rowwise_denom(v_new, a);
         if (VEC) {
           const float4* g4 = reinterpret_cast<const float4*>(g);
           float4* p4 = reinterpret_cast<float4*>(p);
@@ -642,13 +660,33 @@ size_t smore_unique_rows_workspace_bytes(size_t n_table_rows) {
 }  // extern "C"
 
 namespace smore {
-// Shared by smore_unique_rows and the owner side of the sharded update (peer_kernels.cu), whose number
-// of ids is only known on the device: with n_dev != nullptr the first min(n, *n_dev) ids count.
-int unique_rows_impl(const int64_t* idx, size_t n, const int32_t* n_dev, size_t n_table_rows, int64_t* uniq,
-                     int32_t* inverse, int32_t* counts, int32_t* n_unique, void* workspace, size_t workspace_bytes,
-                     cudaStream_t st) {
+
+static int launch_unique(const IdLists& ids, size_t n, const int32_t* n_dev, size_t n_table_rows, int64_t* uniq,
+                         int32_t* inverse, int32_t* counts, int32_t* n_unique, float* g_rows, size_t width,
+                         const UniqueWorkspace& w, cudaStream_t st) {
+  // the bitmap and the finished-blocks counter behind it
+  if (cudaMemsetAsync(w.bitmap, 0, (w.nwords + 1) * sizeof(uint32_t), st) != cudaSuccess)
+    return fail(SMORE_ERR_CUDA, "unique_rows: cudaMemsetAsync failed");
+  if (w.nwords <= kLocalWords) {
+    // every CTA merges its whole bitmap at the end: few CTAs with many ids each
+    const int grid = (int)std::max<size_t>(1, std::min<size_t>((n + 1023) / 1024, (size_t)sm_count()));
+    unique_mark_kernel<true><<<grid, 256, w.nwords * sizeof(uint32_t), st>>>(ids, n, n_dev, n_table_rows, w.nwords, w.bitmap,
+                                                                             counts);
+  } else {
+    unique_mark_kernel<false><<<thread_grid(n), 256, 0, st>>>(ids, n, n_dev, n_table_rows, w.nwords, w.bitmap, counts);
+  }
+  unique_prefix_kernel<<<(unsigned)w.nblocks, kScanThreads, 0, st>>>(w.bitmap, w.nwords, w.wordprefix, w.blocksum, w.nblocks,
+                                                                     w.done, n_unique);
+  unique_assign_kernel<<<thread_grid(n), 256, 0, st>>>(ids, n, n_dev, n_table_rows, w.bitmap, w.wordprefix, w.blocksum, uniq,
+                                                       inverse, counts, n_unique, g_rows, width);
+  return check_launch("unique_rows kernels", 3);
+}
+
+static int unique_lists(const IdLists& ids, size_t n, const int32_t* n_dev, size_t n_table_rows, int64_t* uniq,
+                        int32_t* inverse, int32_t* counts, int32_t* n_unique, float* g_rows, size_t width,
+                        void* workspace, size_t workspace_bytes, cudaStream_t st) {
   if (!n_unique) return fail(SMORE_ERR_NULL, "unique_rows: n_unique is NULL");
-  if (n && (!idx || !uniq || !inverse || !counts)) return fail(SMORE_ERR_NULL, "unique_rows: NULL pointer");
+  if (n && (!uniq || !inverse || !counts)) return fail(SMORE_ERR_NULL, "unique_rows: NULL pointer");
   if (n_table_rows == 0 || n_table_rows > ((size_t)1 << 36))
     return fail(SMORE_ERR_BAD_SHAPE, "unique_rows: n_table_rows out of range");
   if (n > ((size_t)1 << 31) - 1) return fail(SMORE_ERR_TOO_LARGE, "unique_rows: more than 2^31-1 ids");
@@ -658,28 +696,42 @@ int unique_rows_impl(const int64_t* idx, size_t n, const int32_t* n_dev, size_t 
   if (workspace_bytes < w.bytes)
     return fail(SMORE_ERR_WORKSPACE, "unique_rows: workspace has %zu bytes, %zu needed", workspace_bytes,
                 w.bytes);
-  if (n_dev == nullptr && n > 0 && n <= (size_t)kSmallUniqueMax && n_table_rows >= ((size_t)1 << 18)) {
+  if (g_rows && (width & 3) == 0 && !aligned16(g_rows))
+    return fail(SMORE_ERR_BAD_SHAPE, "unique_rows: g_rows must be 16-byte aligned");
+  if (n == 0) {
+    if (cudaMemsetAsync(n_unique, 0, 2 * sizeof(int32_t), st) != cudaSuccess)
+      return fail(SMORE_ERR_CUDA, "unique_rows: cudaMemsetAsync failed");
+    return check_launch("unique_rows memset", 0);
+  }
+  if (n_dev == nullptr && n <= (size_t)kSmallUniqueMax && n_table_rows >= ((size_t)1 << 18)) {
     // few ids over a large id space: sort them in one CTA instead of scanning a bitmap of the space
     int P = 32;
     while ((size_t)P < n) P <<= 1;
     unique_small_kernel<<<1, kSmallUniqueThreads, (size_t)P * sizeof(unsigned long long), st>>>(
-        idx, (int)n, n_table_rows, P, uniq, inverse, counts, n_unique);
-    return check_launch("unique_small_kernel");
+        ids, (int)n, n_table_rows, P, uniq, inverse, counts, n_unique);
+    if (int rc = check_launch("unique_small_kernel")) return rc;
+    return g_rows ? smore_zero_shared_rows(g_rows, counts, n_unique, n, width, st) : SMORE_OK;
   }
-  if (cudaMemsetAsync(n_unique, 0, 2 * sizeof(int32_t), st) != cudaSuccess)
-    return fail(SMORE_ERR_CUDA, "unique_rows: cudaMemsetAsync failed");
-  if (n == 0) return check_launch("unique_rows memset", 0);
-  if (cudaMemsetAsync(w.bitmap, 0, w.nwords * sizeof(uint32_t), st) != cudaSuccess ||
-      cudaMemsetAsync(counts, 0, n * sizeof(int32_t), st) != cudaSuccess)
-    return fail(SMORE_ERR_CUDA, "unique_rows: cudaMemsetAsync failed");
-  unique_mark_kernel<<<thread_grid(n), 256, 0, st>>>(idx, n, n_dev, n_table_rows, w.bitmap, n_unique);
-  unique_blocksum_kernel<<<(unsigned)w.nblocks, kScanThreads, 0, st>>>(w.bitmap, w.nwords, w.blocksum);
-  unique_scan_blocks_kernel<<<1, 1024, 0, st>>>(w.blocksum, w.nblocks, n_unique);
-  unique_wordprefix_kernel<<<(unsigned)w.nblocks, kScanThreads, 0, st>>>(w.bitmap, w.nwords, w.blocksum,
-                                                                         w.wordprefix);
-  unique_assign_kernel<<<thread_grid(n), 256, 0, st>>>(idx, n, n_dev, n_table_rows, w.bitmap, w.wordprefix, uniq,
-                                                        inverse, counts);
-  return check_launch("unique_rows kernels", 5);
+  return launch_unique(ids, n, n_dev, n_table_rows, uniq, inverse, counts, n_unique, g_rows, width, w, st);
+}
+
+static IdLists one_list(const int64_t* idx, size_t n) {
+  IdLists ids;
+  for (int i = 0; i < kIdLists; ++i) {
+    ids.ptr[i] = idx;
+    ids.end[i] = n;
+  }
+  return ids;
+}
+
+// Shared by smore_unique_rows and the owner side of the sharded update (peer_kernels.cu), whose number
+// of ids is only known on the device: with n_dev != nullptr the first min(n, *n_dev) ids count.
+int unique_rows_impl(const int64_t* idx, size_t n, const int32_t* n_dev, size_t n_table_rows, int64_t* uniq,
+                     int32_t* inverse, int32_t* counts, int32_t* n_unique, void* workspace, size_t workspace_bytes,
+                     cudaStream_t st) {
+  if (n && !idx) return fail(SMORE_ERR_NULL, "unique_rows: NULL pointer");
+  return unique_lists(one_list(idx, n), n, n_dev, n_table_rows, uniq, inverse, counts, n_unique, nullptr, 0, workspace,
+                      workspace_bytes, st);
 }
 }  // namespace smore
 
@@ -690,6 +742,25 @@ int smore_unique_rows(const int64_t* idx, size_t n, size_t n_table_rows, int64_t
                       void* stream) {
   return unique_rows_impl(idx, n, nullptr, n_table_rows, uniq, inverse, counts, n_unique, workspace, workspace_bytes,
                           (cudaStream_t)stream);
+}
+
+int smore_step_rows(const int64_t* const* lists, const size_t* list_sizes, size_t n_lists, size_t n_table_rows,
+                    int64_t* uniq, int32_t* inverse, int32_t* counts, int32_t* n_unique, float* g_rows, size_t width,
+                    void* workspace, size_t workspace_bytes, void* stream) {
+  if (n_lists && (!lists || !list_sizes)) return fail(SMORE_ERR_NULL, "step_rows: NULL pointer");
+  if (!g_rows || !width) return fail(SMORE_ERR_NULL, "step_rows: g_rows is NULL or width is 0");
+  if (n_lists > (size_t)kIdLists) return fail(SMORE_ERR_TOO_LARGE, "step_rows: at most %d id lists", kIdLists);
+  IdLists ids = one_list(nullptr, 0);
+  size_t n = 0;
+  for (size_t i = 0; i < n_lists; ++i) {
+    if (list_sizes[i] && !lists[i]) return fail(SMORE_ERR_NULL, "step_rows: list %zu is NULL", i);
+    n += list_sizes[i];
+    ids.ptr[i] = lists[i];
+    ids.end[i] = n;
+  }
+  for (size_t i = n_lists; i < (size_t)kIdLists; ++i) ids.end[i] = n;
+  return unique_lists(ids, n, nullptr, n_table_rows, uniq, inverse, counts, n_unique, g_rows, width, workspace,
+                      workspace_bytes, (cudaStream_t)stream);
 }
 
 int smore_zero_shared_rows(float* g_rows, const int32_t* slot_count, const int32_t* n_unique, size_t capacity,
@@ -826,7 +897,7 @@ namespace smore {
 constexpr size_t kStaticUniqueMaxRows = SMORE_UNIQUE_STATIC_MAX_ROWS;
 constexpr size_t kStaticUniqueWords = kStaticUniqueMaxRows / 32;
 constexpr size_t kStaticUniqueBytes =
-    2 * kStaticUniqueWords * sizeof(uint32_t) + ((kStaticUniqueWords / kWordsPerBlock) * sizeof(uint32_t) + 255) / 256 * 256;
+    2 * kStaticUniqueWords * sizeof(uint32_t) + 256 + round256((kStaticUniqueWords / kWordsPerBlock) * sizeof(uint32_t));
 
 static __device__ __align__(256) unsigned char g_unique_scratch[kStaticUniqueBytes];
 
@@ -872,19 +943,11 @@ extern "C" int smore_unique_rows_static(const int64_t* idx, size_t n, size_t n_t
   const UniqueWorkspace w = carve_unique_workspace(scratch, n_table_rows);
   if (w.bytes > kStaticUniqueBytes) return fail(SMORE_ERR_WORKSPACE, "unique_rows_static: scratch layout overflow");
   cudaStream_t st = (cudaStream_t)stream;
-  // the array still holds the previous call's bitmap: everything that must start at zero is cleared here
-  if (cudaMemsetAsync(n_unique, 0, 2 * sizeof(int32_t), st) != cudaSuccess)
-    return fail(SMORE_ERR_CUDA, "unique_rows_static: cudaMemsetAsync failed");
-  if (n == 0) return check_launch("unique_rows_static memset", 0);
-  if (cudaMemsetAsync(w.bitmap, 0, w.nwords * sizeof(uint32_t), st) != cudaSuccess ||
-      cudaMemsetAsync(counts, 0, n * sizeof(int32_t), st) != cudaSuccess)
-    return fail(SMORE_ERR_CUDA, "unique_rows_static: cudaMemsetAsync failed");
-  unique_mark_kernel<<<thread_grid(n), 256, 0, st>>>(idx, n, nullptr, n_table_rows, w.bitmap, n_unique);
-  unique_blocksum_kernel<<<(unsigned)w.nblocks, kScanThreads, 0, st>>>(w.bitmap, w.nwords, w.blocksum);
-  unique_scan_blocks_kernel<<<1, 1024, 0, st>>>(w.blocksum, w.nblocks, n_unique);
-  unique_wordprefix_kernel<<<(unsigned)w.nblocks, kScanThreads, 0, st>>>(w.bitmap, w.nwords, w.blocksum,
-                                                                         w.wordprefix);
-  unique_assign_kernel<<<thread_grid(n), 256, 0, st>>>(idx, n, nullptr, n_table_rows, w.bitmap, w.wordprefix, uniq,
-                                                        inverse, counts);
-  return check_launch("unique_rows_static kernels", 5);
+  if (n == 0) {
+    if (cudaMemsetAsync(n_unique, 0, 2 * sizeof(int32_t), st) != cudaSuccess)
+      return fail(SMORE_ERR_CUDA, "unique_rows_static: cudaMemsetAsync failed");
+    return check_launch("unique_rows_static memset", 0);
+  }
+  // (the array still holds the previous call's bitmap: launch_unique clears what must start at zero)
+  return launch_unique(one_list(idx, n), n, nullptr, n_table_rows, uniq, inverse, counts, n_unique, nullptr, 0, w, st);
 }
