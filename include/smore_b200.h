@@ -223,6 +223,15 @@ SMORE_API int smore_unique_rows(const int64_t* idx, size_t n, size_t n_table_row
                       int32_t* inverse, int32_t* counts, int32_t* n_unique, void* workspace,
                       size_t workspace_bytes, void* stream);
 
+/* smore_unique_rows over up to 8 id lists taken one after the other (a step's lookups: their ids need not be
+ * copied together first), with the compact gradient rows that several positions contribute to cleared on
+ * the way (what smore_zero_shared_rows does).  `lists` and `list_sizes` are host arrays; outputs and
+ * workspace as for smore_unique_rows with n = the sum of the sizes; g_rows [n, width]. */
+SMORE_API int smore_step_rows(const int64_t* const* lists, const size_t* list_sizes, size_t n_lists, size_t n_table_rows,
+                    int64_t* uniq, int32_t* inverse, int32_t* counts, int32_t* n_unique, float* g_rows,
+                    size_t width, void* workspace, size_t workspace_bytes, void* stream);
+
+
 /* smore_unique_rows for callers that cannot provide scratch memory.  (No counterpart in the
  * reference: it exists for hosts that cannot allocate when they call — a server whose memory
  * manager reserved the whole GPU at start-up, so that a later cudaMalloc fails, or a steady-state
@@ -291,6 +300,15 @@ SMORE_API int smore_sparse_update_rows(int opt_id, float* table, float* m, float
  *   - SMORE_ERR_BAD_SHAPE when the shape is not covered (then nothing was enqueued: call the
  *     ordinary backward). */
 SMORE_API int smore_rows_backward_fused_adam(int dist_id, const float* gout0, const float* gout1, float* table,
+                                   const int64_t* idx, size_t n_table_rows, const float* first,
+                                   const float* second, const int32_t* slot, const int32_t* slot_count,
+                                   float* g_rows, float* g_first, float* g_second, size_t branches,
+                                   size_t bsize, size_t num, size_t dim, float* m, float* v, int64_t* uniq,
+                                   double lr, double beta1, double beta2, double eps, int64_t step,
+                                   const float* step_scalars, void* stream);
+/* The same with a full second moment: v is [n_table_rows, mul*dim] like m.  Covers dims up to 1024 of any
+ * row length (SMORE_ERR_BAD_SHAPE otherwise). */
+SMORE_API int smore_rows_backward_fused_adam_full(int dist_id, const float* gout0, const float* gout1, float* table,
                                    const int64_t* idx, size_t n_table_rows, const float* first,
                                    const float* second, const int32_t* slot, const int32_t* slot_count,
                                    float* g_rows, float* g_first, float* g_second, size_t branches,

@@ -94,7 +94,7 @@ struct Lookup {
 struct StepPlan {
   std::vector<std::shared_ptr<Lookup>> lookups;
   int64_t n = 0;
-  Tensor idx_all, uniq, slot, counts, n_unique, g_rows;
+  Tensor uniq, slot, counts, n_unique, g_rows;
 
   const int32_t* slot_of(const Lookup& lk) const { return (const int32_t*)slot.data_ptr() + lk.offset; }
   const int32_t* counts_ptr() const { return (const int32_t*)counts.data_ptr(); }
@@ -152,18 +152,27 @@ struct RowCore {
 
   std::shared_ptr<StepPlan> build_plan(std::vector<std::shared_ptr<Lookup>> lookups) {
     auto p = std::make_shared<StepPlan>();
-    std::vector<Tensor> ids;
+    std::vector<const int64_t*> ids;
+    std::vector<size_t> sizes;
+    std::vector<Tensor> tensors;
     for (auto& lk : lookups) {
       lk->offset = p->n;
       lk->plan = p;
       p->n += lk->n;
-      ids.push_back(lk->idx);
+      ids.push_back((const int64_t*)lk->idx.data_ptr());
+      sizes.push_back((size_t)lk->n);
+      tensors.push_back(lk->idx);
     }
     p->lookups = std::move(lookups);
     c10::cuda::CUDAGuard guard(table.device());
     at::AutoDispatchBelowADInplaceOrView below;
-    p->idx_all = ids.size() == 1 ? ids[0] : at::cat(ids);
-    const auto i64 = p->idx_all.options(), i32 = i64.dtype(at::kInt);
+    Tensor all;
+    if (ids.size() > 8) {       // more lists than one call takes
+      all = at::cat(tensors);
+      ids = {(const int64_t*)all.data_ptr()};
+      sizes = {(size_t)p->n};
+    }
+    const auto i64 = table.options().dtype(at::kLong), i32 = table.options().dtype(at::kInt);
     p->uniq = at::empty({p->n}, i64);
     p->slot = at::empty({p->n}, i32);
     p->counts = at::empty({p->n}, i32);
@@ -172,14 +181,10 @@ struct RowCore {
     if (!workspace.defined())
       workspace = at::empty({(int64_t)smore_unique_rows_workspace_bytes((size_t)rows())}, table.options().dtype(at::kByte));
     Timed timed("unique_rows");
-    void* st = stream_of(table);
-    check(smore_unique_rows((const int64_t*)p->idx_all.data_ptr(), (size_t)p->n, (size_t)rows(), (int64_t*)p->uniq.data_ptr(),
-                            (int32_t*)p->slot.data_ptr(), (int32_t*)p->counts.data_ptr(), (int32_t*)p->n_unique.data_ptr(),
-                            workspace.data_ptr(), (size_t)workspace.numel(), st),
-          "smore_unique_rows");
-    check(smore_zero_shared_rows(fmut(p->g_rows), p->counts_ptr(), (const int32_t*)p->n_unique.data_ptr(), (size_t)p->n,
-                                 (size_t)width(), st),
-          "smore_zero_shared_rows");
+    check(smore_step_rows(ids.data(), sizes.data(), ids.size(), (size_t)rows(), (int64_t*)p->uniq.data_ptr(),
+                          (int32_t*)p->slot.data_ptr(), (int32_t*)p->counts.data_ptr(), (int32_t*)p->n_unique.data_ptr(),
+                          fmut(p->g_rows), (size_t)width(), workspace.data_ptr(), (size_t)workspace.numel(), stream_of(table)),
+          "smore_step_rows");
     return p;
   }
 
@@ -325,7 +330,8 @@ struct FusedLaunch {
 
   bool run() {
     const bool dev = core->step_dev.defined();
-    const int rc = smore_rows_backward_fused_adam(
+    auto fused = core->squeeze ? smore_rows_backward_fused_adam : smore_rows_backward_fused_adam_full;
+    const int rc = fused(
         dist_id, fptr(g0), fptr(g1), fmut(core->table), (const int64_t*)lk->idx.data_ptr(), (size_t)core->rows(), fptr(first),
         fptr(second), plan->slot_of(*lk), plan->counts_ptr(), fmut(plan->g_rows), fmut(g_first), fmut(g_second),
         (size_t)branches, (size_t)bsize, (size_t)num, (size_t)dim, fmut(core->m), fmut(core->v),
@@ -973,7 +979,6 @@ PYBIND11_MODULE(_host, mod) {
   py::class_<StepPlan, std::shared_ptr<StepPlan>>(mod, "StepPlan")
       .def_readonly("lookups", &StepPlan::lookups)
       .def_readonly("n", &StepPlan::n)
-      .def_readonly("idx_all", &StepPlan::idx_all)
       .def_readonly("uniq", &StepPlan::uniq)
       .def_readonly("slot", &StepPlan::slot)
       .def_readonly("counts", &StepPlan::counts)

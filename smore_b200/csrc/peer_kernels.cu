@@ -431,7 +431,8 @@ template <int NCH, bool ROWWISE>
 __device__ __forceinline__ void adam_row(float4 (&g)[NCH], float4 (&p)[NCH], float4 (&m)[NCH], float4 (&v)[NCH],
                                          float4* p4, float4* m4, float4* v4, int64_t row, int lane, int w4,
                                          const UpdateArgs& a) {
-  float denom = 0.f, v_old = 0.f, v_new = 0.f;
+  RowDenom denom = {1.f, 1.f};
+  float v_old = 0.f, v_new = 0.f;
   if (ROWWISE) {
     v_old = a.v[row];
     float s = 0.f;
@@ -440,7 +441,7 @@ __device__ __forceinline__ void adam_row(float4 (&g)[NCH], float4 (&p)[NCH], flo
       if (lane + 32 * j < w4) s += g[j].x * g[j].x + g[j].y * g[j].y + g[j].z * g[j].z + g[j].w * g[j].w;
     const float g2mean = warp_sum(s) / (float)a.width;
     v_new = v_old * a.beta2 + g2mean * a.omb2;
-    denom = sqrtf(v_new) / a.sqrt_bc2 + a.eps;
+    denom = rowwise_denom(v_new, a);
   }
 #pragma unroll
   for (int j = 0; j < NCH; ++j) {

@@ -269,7 +269,7 @@ class EmbeddingOptimizer(object):
         self.lazy_names = tuple(lazy_names)
         self._local_state = {}
         self.core = _lib.host().RowCore(self.table, self.dummy_tensor, _lib.OPT_IDS[self.opt_name], self.squeeze,
-                                        self.opt_name == "adam" and self.squeeze and not self.share_optim_stats)
+                                        self.opt_name == "adam" and not self.share_optim_stats)
         if self.share_optim_stats:
             for name in self.state_names:
                 if not hasattr(sp_embed, name):
@@ -313,10 +313,9 @@ class EmbeddingOptimizer(object):
         one distance op may then have the rows that only ONE position of the step touches updated
         inside that op's backward kernel (smore_rows_backward_fused_adam) instead of writing their
         gradient out for apply_grad to read back; the result is the same update.  Only the Adam
-        optimizer with a row-wise second moment does this; others ignore the call.  A step that
-        announced a learning rate must end with apply_grad of the same value (some rows have
-        already moved)."""
-        if self.opt_name != "adam" or not self.squeeze:
+        optimizer does this; others ignore the call.  A step that announced a learning rate must end
+        with apply_grad of the same value (some rows have already moved)."""
+        if self.opt_name != "adam":
             return
         self.core.announce(float(lr), *self._moments())
 
