@@ -2270,7 +2270,9 @@ extern "C" int smore_rows_status(int* status);         // rows_kernels.cu (likew
 extern "C" int smore_query_status(int* status);        // query_kernels.cu (likewise)
 extern "C" int smore_shared_status(int* status);       // shared_kernels.cu (likewise)
 extern "C" int smore_cell_status(int* status);         // cell_kernels.cu (likewise)
+extern "C" int smore_split_status(int* status);        // gemm_split_sm100.cu (likewise)
 extern "C" int smore_shared_status_clear(void);
+extern "C" int smore_split_status_clear(void);
 extern "C" int smore_cell_status_clear(void);
 extern "C" int smore_peer_status_clear(void);
 extern "C" int smore_rows_status_clear(void);
@@ -2283,11 +2285,12 @@ int smore_async_status(int* status) {
   if (e != cudaSuccess) return fail(SMORE_ERR_CUDA, "async_status: %s", cudaGetErrorString(e));
   if (int rc = smore_peer_async_status(&peer)) return rc;   // the other files' kernels keep their own words
   if (int rc = smore_rows_status(&rows)) return rc;
-  int query = 0, shared = 0, cell = 0;
+  int query = 0, shared = 0, cell = 0, split = 0;
   if (int rc = smore_query_status(&query)) return rc;
   if (int rc = smore_shared_status(&shared)) return rc;
   if (int rc = smore_cell_status(&cell)) return rc;
-  *status = v | shared | cell | ((peer & 1) ? kStatusPeerWait : 0) | (peer & ~1) | rows | query;
+  if (int rc = smore_split_status(&split)) return rc;
+  *status = v | shared | cell | split | ((peer & 1) ? kStatusPeerWait : 0) | (peer & ~1) | rows | query;
   return SMORE_OK;
 }
 
@@ -2300,6 +2303,7 @@ int smore_async_status_clear(void) {
   if (int rc = smore_query_status_clear()) return rc;
   if (int rc = smore_shared_status_clear()) return rc;
   if (int rc = smore_cell_status_clear()) return rc;
+  if (int rc = smore_split_status_clear()) return rc;
   return smore_rows_status_clear();
 }
 

@@ -8,17 +8,17 @@
 //     g_query[B, W] = g[B, K]     . cand[K, W]
 //     g_cand[K, W]  = g[B, K]^T   . query[B, W]
 // W is the row length (dim for DistMult; 2*dim for ComplEx, with the query laid out [re | im] like
-// the entity rows).  The kernels are CUTLASS 3.x sm100 templates instantiated here: TMA loads,
-// tcgen05.mma with TMEM accumulators, one SM per 128 x 128 tile (cluster 1x1x1), fp32 in / fp32 out,
-// in two
-// precisions: TF32 (10-bit mantissa products) and "fast fp32" (each fp32 operand split into three
-// bf16 terms, nine bf16 MMAs per product, fp32-level accuracy).
+// the entity rows).  Two precisions: fp32-level (each fp32 operand split into three bf16 planes, nine bf16
+// products per product: gemm_split_sm100.cu) and TF32 (10-bit mantissa products), whose kernels are CUTLASS
+// 3.x sm100 templates instantiated here: TMA loads, tcgen05.mma with TMEM accumulators, one SM per
+// 128 x 128 tile (cluster 1x1x1), fp32 in / fp32 out.
 //
-// Built only when a CUTLASS header tree is found (see build.py); without it the entry points
-// report SMORE_ERR_BAD_SHAPE and callers use the SIMT tile kernels.
+// The TF32 kernels are built only when a CUTLASS header tree is found (see build.py); without it the entry
+// points report SMORE_ERR_BAD_SHAPE and callers use the SIMT tile kernels.
 #include <cuda_runtime.h>
 
 #include "common.cuh"
+#include "gemm_split.cuh"
 
 extern "C" int smore_dot_available(void);
 
@@ -43,14 +43,13 @@ using namespace cute;
 enum { kOk = 0, kBadShape = 1, kWorkspace = 2, kCuda = 3 };
 
 // One SM per 128 x 128 tile, cluster 1 x 1 x 1.
-template <class LayoutA, class LayoutB, bool kFast>
+template <class LayoutA, class LayoutB>
 struct DotGemm {
   using Acc = float;
   using LayoutC = cutlass::layout::RowMajor;
   using Tile = Shape<_128, _128, _32>;
   using Cluster = Shape<_1, _1, _1>;
-  using Schedule = cute::conditional_t<kFast, cutlass::gemm::KernelTmaWarpSpecialized1SmFastFP32Sm100,
-                                       cutlass::gemm::KernelTmaWarpSpecialized1SmSm100>;
+  using Schedule = cutlass::gemm::KernelTmaWarpSpecialized1SmSm100;
   using Epi = typename cutlass::epilogue::collective::CollectiveBuilder<
       cutlass::arch::Sm100, cutlass::arch::OpClassTensorOp, Tile, Cluster,
       cutlass::epilogue::collective::EpilogueTileAuto, Acc, Acc, float, LayoutC, 4, float, LayoutC, 4,
@@ -66,10 +65,10 @@ struct DotGemm {
 // D[M, N] = A . B with A(m, k), B(k, n) in the given layouts ("column-major B" = an [N, K] row-major
 // array).  need != nullptr: only report the workspace size.  Returns one of the codes above;
 // *ws_needed receives the workspace size when that is what is missing.
-template <class LayoutA, class LayoutB, bool kFast>
+template <class LayoutA, class LayoutB>
 static int run_gemm(const float* A, const float* B, float* D, int M, int N, int K, void* ws, size_t ws_bytes,
                     cudaStream_t st, size_t* need) {
-  using Gemm = typename DotGemm<LayoutA, LayoutB, kFast>::Gemm;
+  using Gemm = typename DotGemm<LayoutA, LayoutB>::Gemm;
   using StrideA = typename Gemm::GemmKernel::StrideA;
   using StrideB = typename Gemm::GemmKernel::StrideB;
   using StrideC = typename Gemm::GemmKernel::StrideC;
@@ -104,7 +103,7 @@ using namespace smore_gemm;
 // on tiles shared by two SMs.  It is optional: when the file sits next to this library it is loaded
 // on first use and takes the products with at least 256 output rows; without it everything runs on
 // the one-SM tiles.
-typedef int (*TwoSmRun)(int layout, int fast, const float* A, const float* B, float* D, int M, int N, int K, void* ws,
+typedef int (*TwoSmRun)(int layout, const float* A, const float* B, float* D, int M, int N, int K, void* ws,
                         size_t ws_bytes, void* stream, size_t* need);
 static TwoSmRun g_two_sm = nullptr;
 static std::once_flag g_two_sm_once;
@@ -135,27 +134,11 @@ static int gemm_status(int code, int M, int N, int K) {
 enum { kLayoutRowCol = 0, kLayoutRowRow = 1, kLayoutColRow = 2 };
 
 template <class LayoutA, class LayoutB, int kLayout>
-static int run_precision(int precision, const float* A, const float* B, float* D, int M, int N, int K, void* ws,
-                         size_t ws_bytes, cudaStream_t st, size_t* need) {
-  if (precision != SMORE_DOT_TF32 && precision != SMORE_DOT_FP32)
-    return fail(SMORE_ERR_BAD_DIST, "unknown dot precision %d", precision);
-  const bool fast = precision == SMORE_DOT_FP32;
-  int code;
-  // Building the tensor maps is a driver call and needs a current context; a thread whose first CUDA call
-  // this is (autograd's) has none until it sets its device.
-  static thread_local int bound = -1;
-  int dev = 0;
-  if (!need && cudaGetDevice(&dev) == cudaSuccess && dev != bound) {
-    if (cudaSetDevice(dev) != cudaSuccess) return fail(SMORE_ERR_CUDA, "dot: cudaSetDevice failed");
-    bound = dev;
-  }
+static int run_tf32(const float* A, const float* B, float* D, int M, int N, int K, void* ws, size_t ws_bytes, cudaStream_t st,
+                    size_t* need) {
   TwoSmRun wide = M >= 256 ? two_sm() : nullptr;
-  if (wide != nullptr) {
-    code = wide(kLayout, fast ? 1 : 0, A, B, D, M, N, K, ws, ws_bytes, st, need);
-  } else {
-    code = fast ? run_gemm<LayoutA, LayoutB, true>(A, B, D, M, N, K, ws, ws_bytes, st, need)
-                : run_gemm<LayoutA, LayoutB, false>(A, B, D, M, N, K, ws, ws_bytes, st, need);
-  }
+  const int code = wide != nullptr ? wide(kLayout, A, B, D, M, N, K, ws, ws_bytes, st, need)
+                                   : run_gemm<LayoutA, LayoutB>(A, B, D, M, N, K, ws, ws_bytes, st, need);
   if (code == kOk && !need) count_launches(1);
   return gemm_status(code, M, N, K);
 }
@@ -191,11 +174,16 @@ int smore_dot_two_sm(void) {
 
 size_t smore_dot_workspace_bytes(size_t B, size_t K, size_t W, int precision) {
 #ifdef SMORE_HAVE_CUTLASS
-  size_t n0 = 0, n1 = 0, n2 = 0;
   if (check_sizes(B, K, W)) return 0;
-  run_precision<RowM, ColM, kLayoutRowCol>(precision, nullptr, nullptr, nullptr, (int)B, (int)K, (int)W, nullptr, 0, nullptr, &n0);
-  run_precision<RowM, RowM, kLayoutRowRow>(precision, nullptr, nullptr, nullptr, (int)B, (int)W, (int)K, nullptr, 0, nullptr, &n1);
-  run_precision<ColM, RowM, kLayoutColRow>(precision, nullptr, nullptr, nullptr, (int)K, (int)W, (int)B, nullptr, 0, nullptr, &n2);
+  if (precision == SMORE_DOT_FP32) {
+    const size_t forward = split_plane_bytes(B, W) + split_plane_bytes(K, W);
+    const size_t backward = split_plane_bytes(B, K) + split_plane_bytes(K, B) + split_plane_bytes(W, K) + split_plane_bytes(W, B);
+    return 1024 + (forward > backward ? forward : backward);
+  }
+  size_t n0 = 0, n1 = 0, n2 = 0;
+  run_tf32<RowM, ColM, kLayoutRowCol>(nullptr, nullptr, nullptr, (int)B, (int)K, (int)W, nullptr, 0, nullptr, &n0);
+  run_tf32<RowM, RowM, kLayoutRowRow>(nullptr, nullptr, nullptr, (int)B, (int)W, (int)K, nullptr, 0, nullptr, &n1);
+  run_tf32<ColM, RowM, kLayoutColRow>(nullptr, nullptr, nullptr, (int)K, (int)W, (int)B, nullptr, 0, nullptr, &n2);
   size_t n = n0 > n1 ? n0 : n1;
   n = n > n2 ? n : n2;
   return n < 256 ? 256 : n;
@@ -205,14 +193,52 @@ size_t smore_dot_workspace_bytes(size_t B, size_t K, size_t W, int precision) {
 #endif
 }
 
+// Checks common to both passes; binds the calling thread to its device.
+static int dot_check(const char* what, size_t B, size_t K, size_t W, int precision) {
+  if (int rc = check_sizes(B, K, W)) return rc;
+  if (precision != SMORE_DOT_TF32 && precision != SMORE_DOT_FP32)
+    return fail(SMORE_ERR_BAD_DIST, "unknown dot precision %d", precision);
+  if (precision == SMORE_DOT_FP32 && ((B | K | W) & 3))
+    return fail(SMORE_ERR_BAD_SHAPE, "%s: sizes must be multiples of 4 (B=%zu K=%zu W=%zu)", what, B, K, W);
+  // Building the tensor maps is a driver call and needs a current context; a thread whose first CUDA call
+  // this is (autograd's) has none until it sets its device.
+  static thread_local int bound = -1;
+  int dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && dev != bound) {
+    if (cudaSetDevice(dev) != cudaSuccess) return fail(SMORE_ERR_CUDA, "dot: cudaSetDevice failed");
+    bound = dev;
+  }
+  return SMORE_OK;
+}
+
+// consecutive plane buffers of the caller's workspace
+struct Planes {
+  unsigned char* at;
+  explicit Planes(void* ws) : at(reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ws) + 1023) & ~(uintptr_t)1023)) {}
+  void* take(size_t rows, size_t k) {
+    void* p = at;
+    at += split_plane_bytes(rows, k);
+    return p;
+  }
+};
+
 int smore_dot_forward_shared(const float* cand, const float* query, float* dst, size_t B, size_t K, size_t W,
                              int precision, void* workspace, size_t workspace_bytes, void* stream) {
   if (!cand || !query || !dst) return fail(SMORE_ERR_NULL, "dot_forward_shared: NULL pointer");
-  if (int rc = check_sizes(B, K, W)) return rc;
 #ifdef SMORE_HAVE_CUTLASS
-  return run_precision<RowM, ColM, kLayoutRowCol>(precision, query, cand, dst, (int)B, (int)K, (int)W, workspace, workspace_bytes,
-                                   (cudaStream_t)stream, nullptr);
+  if (int rc = dot_check("dot_forward_shared", B, K, W, precision)) return rc;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (precision == SMORE_DOT_FP32) {
+    if (!workspace || workspace_bytes < smore_dot_workspace_bytes(B, K, W, precision)) return gemm_status(kWorkspace, 0, 0, 0);
+    Planes ws(workspace);
+    void *q = ws.take(B, W), *c = ws.take(K, W);
+    if (int rc = split_planes(query, B, W, q, nullptr, st)) return rc;
+    if (int rc = split_planes(cand, K, W, c, nullptr, st)) return rc;
+    return split_gemm(q, c, dst, B, K, W, st);
+  }
+  return run_tf32<RowM, ColM, kLayoutRowCol>(query, cand, dst, (int)B, (int)K, (int)W, workspace, workspace_bytes, st, nullptr);
 #else
+  if (int rc = check_sizes(B, K, W)) return rc;
   (void)precision; (void)workspace; (void)workspace_bytes; (void)stream;
   return fail(SMORE_ERR_BAD_SHAPE, "library built without the tensor-core GEMM path");
 #endif
@@ -222,17 +248,26 @@ int smore_dot_backward_shared(const float* gout, const float* cand, const float*
                               float* g_query, size_t B, size_t K, size_t W, int precision, void* workspace,
                               size_t workspace_bytes, void* stream) {
   if (!gout || !cand || !query || !g_cand || !g_query) return fail(SMORE_ERR_NULL, "dot_backward_shared: NULL pointer");
-  if (int rc = check_sizes(B, K, W)) return rc;
 #ifdef SMORE_HAVE_CUTLASS
+  if (int rc = dot_check("dot_backward_shared", B, K, W, precision)) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  // g_query[B, W] = gout[B, K] . cand[K, W]
-  if (int rc = run_precision<RowM, RowM, kLayoutRowRow>(precision, gout, cand, g_query, (int)B, (int)W, (int)K, workspace,
-                                         workspace_bytes, st, nullptr))
+  // g_query[B, W] = gout[B, K] . cand[K, W];  g_cand[K, W] = gout^T[K, B] . query[B, W]
+  if (precision == SMORE_DOT_FP32) {
+    if (!workspace || workspace_bytes < smore_dot_workspace_bytes(B, K, W, precision)) return gemm_status(kWorkspace, 0, 0, 0);
+    Planes ws(workspace);
+    void *g = ws.take(B, K), *gt = ws.take(K, B), *ct = ws.take(W, K), *qt = ws.take(W, B);
+    if (int rc = split_planes(gout, B, K, g, gt, st)) return rc;
+    if (int rc = split_planes(cand, K, W, nullptr, ct, st)) return rc;
+    if (int rc = split_planes(query, B, W, nullptr, qt, st)) return rc;
+    if (int rc = split_gemm(g, ct, g_query, B, W, K, st)) return rc;
+    return split_gemm(gt, qt, g_cand, K, W, B, st);
+  }
+  if (int rc = run_tf32<RowM, RowM, kLayoutRowRow>(gout, cand, g_query, (int)B, (int)W, (int)K, workspace, workspace_bytes, st,
+                                                   nullptr))
     return rc;
-  // g_cand[K, W] = gout^T[K, B] . query[B, W]
-  return run_precision<ColM, RowM, kLayoutColRow>(precision, gout, query, g_cand, (int)K, (int)W, (int)B, workspace, workspace_bytes,
-                                   st, nullptr);
+  return run_tf32<ColM, RowM, kLayoutColRow>(gout, query, g_cand, (int)K, (int)W, (int)B, workspace, workspace_bytes, st, nullptr);
 #else
+  if (int rc = check_sizes(B, K, W)) return rc;
   (void)precision; (void)workspace; (void)workspace_bytes; (void)stream;
   return fail(SMORE_ERR_BAD_SHAPE, "library built without the tensor-core GEMM path");
 #endif

@@ -1,0 +1,16 @@
+// fp32-accurate products on the bf16 tensor cores (gemm_split_sm100.cu).
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstddef>
+
+namespace smore {
+
+// bytes of the three bf16 planes of [rows, k]
+size_t split_plane_bytes(size_t rows, size_t k);
+// fp32 [rows, cols] (cols and rows multiples of 4) -> planes of it and / or of its transpose; either may be nullptr
+int split_planes(const float* x, size_t rows, size_t cols, void* plain, void* transposed, cudaStream_t st);
+// D[M, N] = A . B^T from planes of A [M, K] and B [N, K]; N a multiple of 4
+int split_gemm(const void* a_planes, const void* b_planes, float* d, size_t M, size_t N, size_t K, cudaStream_t st);
+
+}  // namespace smore

@@ -1,0 +1,427 @@
+// fp32-accurate matrix products on the bf16 tensor cores, for dot-product scoring against a shared list.
+//
+// Every fp32 operand is split once, ahead of the product, into three bf16 planes whose sum is the operand
+// (8 + 8 + 8 significant bits); the product is the sum of the nine plane products.  A GEMM that splits its
+// operands inside the main loop repeats that work for every tile that reads them and keeps the tensor cores
+// waiting for it: 4096 x 8192 x 1000 ran at 0.49 of the bf16 rate / 9 that way.  Here the main loop only
+// moves bf16 tiles (TMA) and issues tcgen05.mma.
+//
+//   split_planes_kernel   fp32 [rows, cols] -> planes [3][rows][ld] and / or transposed [3][cols][ld_t]; all
+//                         products then have both operands K-major, and one GEMM kernel serves them
+//   split_gemm_kernel     D[M, N] = A . B^T, A planes [3][M][K], B planes [3][N][K]; one 128 x 256 tile per
+//                         CTA at a time, a fixed set of CTAs walks the tiles.  Warp 0 issues the TMA loads,
+//                         warp 1 the MMAs, warps 2..9 own the result.
+//
+// Precision: a tensor-memory accumulator is added to once per 16 products, with truncation.  So that this
+// does not add up over a long reduction, the accumulator holds kChunk of it only and is then added, in fp32
+// with rounding to nearest, to the running sums in the registers of warps 2..9, while the MMAs go on in a
+// second accumulator; within a chunk the products of the small planes come first.
+//
+// Every wait on an mbarrier is bounded; one that runs out sets kStatusCopyWait and lets the CTA finish.
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "bulk_copy.cuh"
+#include "common.cuh"
+#include "gemm_split.cuh"
+
+namespace smore {
+
+static __device__ int g_split_status = 0;
+
+// ----------------------------------------------------------------------------------------
+// planes
+// ----------------------------------------------------------------------------------------
+
+constexpr int kSplitTile = 64;
+
+__device__ __forceinline__ void split3(float x, __nv_bfloat16 (&p)[3]) {
+  p[0] = __float2bfloat16_rn(x);
+  const float r = x - __bfloat162float(p[0]);        // exact
+  p[1] = __float2bfloat16_rn(r);
+  p[2] = __float2bfloat16_rn(r - __bfloat162float(p[1]));
+}
+
+// One 64 x 64 block per CTA.  plain: [3][rows][ld], transposed: [3][cols][ld_t]; either may be nullptr.
+__global__ void __launch_bounds__(256)
+    split_planes_kernel(const float* __restrict__ x, int rows, int cols, __nv_bfloat16* __restrict__ plain, size_t ld,
+                        __nv_bfloat16* __restrict__ transposed, size_t ld_t) {
+  __shared__ float tile[kSplitTile][kSplitTile + 1];
+  const int r0 = blockIdx.y * kSplitTile, c0 = blockIdx.x * kSplitTile;
+  const int t = threadIdx.x;
+  {
+    // 4 floats per thread and pass; cols is a multiple of 4
+    const int c = c0 + (t & 15) * 4;
+    for (int r = t >> 4; r < kSplitTile; r += 16) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r0 + r < rows && c < cols) v = __ldg(reinterpret_cast<const float4*>(x + (size_t)(r0 + r) * cols + c));
+      float* d = &tile[r][(t & 15) * 4];
+      d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
+    }
+  }
+  __syncthreads();
+  // a thread writes two consecutive elements of each plane
+  auto write = [&](__nv_bfloat16* out, size_t stride, size_t plane, int a0, int n_a, int b0, int n_b, bool flip) {
+    const int b = (t & 31) * 2;
+    for (int a = t >> 5; a < kSplitTile; a += 8) {
+      if (a0 + a >= n_a || b0 + b >= n_b) continue;
+      __nv_bfloat16 u[3], v[3];
+      split3(flip ? tile[b][a] : tile[a][b], u);
+      split3(flip ? tile[b + 1][a] : tile[a][b + 1], v);
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        __nv_bfloat162 w;
+        w.x = u[p];
+        w.y = v[p];
+        // (the row pitch is even and at least n_b: the second element of an odd end lands in the padding)
+        *reinterpret_cast<__nv_bfloat162*>(out + p * plane + (size_t)(a0 + a) * stride + b0 + b) = w;
+      }
+    }
+  };
+  if (plain) write(plain, ld, (size_t)rows * ld, r0, rows, c0, cols, false);
+  if (transposed) write(transposed, ld_t, (size_t)cols * ld_t, c0, cols, r0, rows, true);
+}
+
+// ----------------------------------------------------------------------------------------
+// the product
+// ----------------------------------------------------------------------------------------
+
+constexpr int kTileM = 128, kTileN = 256;
+constexpr int kBlockK = 32;                      // reduction per pipeline stage: 64-byte rows, 64-byte swizzle
+constexpr int kChunk = 64;                       // reduction per tensor-memory accumulator
+constexpr int kBlocksPerChunk = kChunk / kBlockK;
+constexpr int kStages = 3;
+constexpr int kPlaneA = kTileM * kBlockK * 2, kPlaneB = kTileN * kBlockK * 2;    // bytes
+constexpr int kStageBytes = 3 * (kPlaneA + kPlaneB);                             // 72 KB
+constexpr int kGemmThreads = 320;
+constexpr int kGemmSmem = kStages * kStageBytes + 1024 /* alignment */;
+
+struct GemmArgs {
+  float* d;              // [M, N] row-major
+  int M, N;
+  int k_blocks;          // stages of the whole reduction
+  int splits;            // parts the reduction is cut into; > 1: parts are added into a zeroed d
+  int tiles_m, tiles_n;
+};
+
+__device__ __forceinline__ bool wait_bar(uint64_t* bar, unsigned parity) {
+  if (bulk::barrier_wait(bar, parity)) return true;
+  atomicOr(&g_split_status, kStatusCopyWait);
+  return false;
+}
+
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+          bulk::smem_addr(dst)),
+      "l"(map), "r"(x), "r"(y), "r"(z), "r"(bulk::smem_addr(bar))
+      : "memory");
+}
+
+// shared-memory descriptor of a K-major operand tile with 64-byte rows: 64-byte swizzle, 8-row groups 512 B apart
+__device__ __forceinline__ uint64_t operand_desc(uint32_t smem) {
+  return (uint64_t)((smem & 0x3FFFF) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(512 >> 4) << 32) | ((uint64_t)1 << 46) |
+         ((uint64_t)4 << 61);
+}
+
+__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(a), "l"(b), "r"(idesc), "r"((unsigned)accumulate)
+      : "memory");
+}
+
+__device__ __forceinline__ void mma_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bulk::smem_addr(bar))
+               : "memory");
+}
+
+__device__ __forceinline__ void barrier_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bulk::smem_addr(bar)) : "memory");
+}
+
+// 32 consecutive columns of this warp's 32 tensor-memory lanes
+__device__ __forceinline__ void tmem_load32(uint32_t addr, float (&v)[32]) {
+  uint32_t r[32];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]),
+        "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]),
+        "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(addr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// the part of the work item `item` covers: tile and range of stages
+struct Item {
+  int m0, n0, k_begin, k_end;
+};
+__device__ __forceinline__ Item item_of(const GemmArgs& g, int item) {
+  // parts outermost, then tiles row by row of B's tiles: CTAs that run together share operand rows in L2
+  const int tiles = g.tiles_m * g.tiles_n;
+  const int part = item / tiles, t = item - part * tiles;
+  const int tn = t / g.tiles_m, tm = t - tn * g.tiles_m;
+  // parts are whole chunks
+  const int chunks = (g.k_blocks + kBlocksPerChunk - 1) / kBlocksPerChunk;
+  const int per = (chunks + g.splits - 1) / g.splits;
+  return {tm * kTileM, tn * kTileN, min(g.k_blocks, part * per * kBlocksPerChunk),
+          min(g.k_blocks, (part + 1) * per * kBlocksPerChunk)};
+}
+
+__global__ void __launch_bounds__(kGemmThreads, 1)
+    split_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, GemmArgs g) {
+  extern __shared__ unsigned char gemm_smem[];
+  __shared__ uint64_t full[kStages], empty[kStages], acc_full[2], acc_empty[2], drained;
+  __shared__ uint32_t tmem_base_sh;
+  unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gemm_smem) + 1023) & ~(uintptr_t)1023);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      bulk::barrier_init(full + s, 1);
+      bulk::barrier_init(empty + s, 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      bulk::barrier_init(acc_full + i, 1);
+      bulk::barrier_init(acc_empty + i, 8);   // one arrival per result warp
+    }
+    bulk::barrier_init(&drained, 1);
+    bulk::fence_barrier_init();
+  }
+  if (warp == 1) {
+    // both accumulators: all 512 columns of the SM's tensor memory (one CTA per SM)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(bulk::smem_addr(&tmem_base_sh)),
+                 "r"(512)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_base_sh;
+  const int items = g.tiles_m * g.tiles_n * g.splits;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int stage = 0;
+      unsigned parity = 0;
+      long long loads = 0;
+      bool ok = true;
+      for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+        const Item it = item_of(g, item);
+        for (int kb = it.k_begin; kb < it.k_end; ++kb) {
+          ok = wait_bar(empty + stage, parity ^ 1u);
+          if (!ok) break;
+          unsigned char* a = ring + (size_t)stage * kStageBytes;
+          bulk::barrier_expect(full + stage, kStageBytes);
+          tma_load_3d(a, &map_a, kb * kBlockK, it.m0, 0, full + stage);
+          tma_load_3d(a + 3 * kPlaneA, &map_b, kb * kBlockK, it.n0, 0, full + stage);
+          ++loads;
+          if (++stage == kStages) {
+            stage = 0;
+            parity ^= 1u;
+          }
+        }
+      }
+      // no copy of this CTA is still in flight when it ends, whatever became of its readers
+      for (long long l = loads > kStages ? loads - kStages : 0; l < loads; ++l)
+        wait_bar(full + l % kStages, (unsigned)(l / kStages) & 1u);
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      // D fp32, A and B bf16, both K-major, N / 8, M / 16
+      constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((kTileN / 8) << 17) | ((kTileM / 16) << 24);
+      int stage = 0, acc = 0;
+      unsigned parity = 0, acc_parity = 0;
+      bool ok = true;
+      for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+        const Item it = item_of(g, item);
+        for (int kb0 = it.k_begin; kb0 < it.k_end && ok; kb0 += kBlocksPerChunk) {
+          ok = wait_bar(acc_empty + acc, acc_parity ^ 1u);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t d = tmem + acc * kTileN;
+          bool first = true;
+          for (int kb = kb0; kb < min(it.k_end, kb0 + kBlocksPerChunk); ++kb) {
+            ok = wait_bar(full + stage, parity);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t a = bulk::smem_addr(ring + (size_t)stage * kStageBytes), b = a + 3 * kPlaneA;
+            // plane products, the smallest first
+            constexpr int kPa[9] = {2, 2, 1, 2, 1, 0, 1, 0, 0}, kPb[9] = {2, 1, 2, 0, 1, 2, 0, 1, 0};
+#pragma unroll
+            for (int t = 0; t < 9; ++t)
+#pragma unroll
+              for (int k = 0; k < kBlockK / 16; ++k) {
+                mma_bf16(d, operand_desc(a + kPa[t] * kPlaneA + k * 32), operand_desc(b + kPb[t] * kPlaneB + k * 32), kIdesc,
+                         !first);
+                first = false;
+              }
+            mma_commit(empty + stage);
+            if (++stage == kStages) {
+              stage = 0;
+              parity ^= 1u;
+            }
+          }
+          mma_commit(acc_full + acc);
+          if (++acc == 2) {
+            acc = 0;
+            acc_parity ^= 1u;
+          }
+        }
+      }
+      mma_commit(&drained);      // nor is a product
+      wait_bar(&drained, 0);
+    }
+  } else {
+    // a warp reads the tensor-memory lanes (result rows) of its quarter, and half of the tile's columns
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
+    const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
+    int acc = 0;
+    unsigned acc_parity = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+      const Item it = item_of(g, item);
+      float sum[kTileN / 2];
+#pragma unroll
+      for (int i = 0; i < kTileN / 2; ++i) sum[i] = 0.f;
+      for (int kb0 = it.k_begin; kb0 < it.k_end; kb0 += kBlocksPerChunk) {
+        ok = wait_bar(acc_full + acc, acc_parity);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int c = 0; c < kTileN / 2; c += 32) {
+          float v[32];
+          tmem_load32(tmem + lanes + acc * kTileN + half * (kTileN / 2) + c, v);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) sum[c + i] += v[i];
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) barrier_arrive(acc_empty + acc);
+        if (++acc == 2) {
+          acc = 0;
+          acc_parity ^= 1u;
+        }
+      }
+      const int m = it.m0 + quarter * 32 + lane, n0 = it.n0 + half * (kTileN / 2);
+      if (ok && m < g.M && it.k_begin < it.k_end) {
+        float* out = g.d + (size_t)m * g.N + n0;
+#pragma unroll
+        for (int c = 0; c < kTileN / 2; c += 4) {
+          if (n0 + c >= g.N) continue;                // N is a multiple of 4
+          const float4 v = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
+          if (g.splits > 1) atomicAdd(reinterpret_cast<float4*>(out + c), v);
+          else *reinterpret_cast<float4*>(out + c) = v;
+        }
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+  }
+}
+
+// ----------------------------------------------------------------------------------------
+// host side
+// ----------------------------------------------------------------------------------------
+
+typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+static EncodeTiled encode_tiled() {
+  static EncodeTiled fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess)
+      p = nullptr;
+    return reinterpret_cast<EncodeTiled>(p);
+  }();
+  return fn;
+}
+
+size_t split_pitch(size_t k) { return (k + 7) & ~(size_t)7; }
+size_t split_plane_bytes(size_t rows, size_t k) { return (3 * rows * split_pitch(k) * 2 + 1023) & ~(size_t)1023; }
+
+int split_planes(const float* x, size_t rows, size_t cols, void* plain, void* transposed, cudaStream_t st) {
+  const dim3 grid((unsigned)((cols + kSplitTile - 1) / kSplitTile), (unsigned)((rows + kSplitTile - 1) / kSplitTile));
+  split_planes_kernel<<<grid, 256, 0, st>>>(x, (int)rows, (int)cols, static_cast<__nv_bfloat16*>(plain), split_pitch(cols),
+                                            static_cast<__nv_bfloat16*>(transposed), split_pitch(rows));
+  return check_launch("split_planes_kernel");
+}
+
+// map of planes [3][rows][pitch(k)]: boxes of kBlockK x box_rows x 3
+static int plane_map(CUtensorMap* map, const void* planes, size_t rows, size_t k, int box_rows) {
+  const size_t pitch = split_pitch(k) * 2;
+  const cuuint64_t dims[3] = {k, rows, 3}, strides[2] = {pitch, pitch * rows};
+  const cuuint32_t box[3] = {(cuuint32_t)kBlockK, (cuuint32_t)box_rows, 3}, ones[3] = {1, 1, 1};
+  EncodeTiled encode = encode_tiled();
+  if (!encode) return fail(SMORE_ERR_CUDA, "dot: cuTensorMapEncodeTiled is not available");
+  const CUresult rc = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(planes), dims, strides, box, ones,
+                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (rc != CUDA_SUCCESS) return fail(SMORE_ERR_CUDA, "dot: cuTensorMapEncodeTiled failed (%d)", (int)rc);
+  return SMORE_OK;
+}
+
+int split_gemm(const void* a_planes, const void* b_planes, float* d, size_t M, size_t N, size_t K, cudaStream_t st) {
+  CUtensorMap map_a, map_b;
+  if (int rc = plane_map(&map_a, a_planes, M, K, kTileM)) return rc;
+  if (int rc = plane_map(&map_b, b_planes, N, K, kTileN)) return rc;
+  GemmArgs g;
+  g.d = d;
+  g.M = (int)M;
+  g.N = (int)N;
+  g.k_blocks = (int)((K + kBlockK - 1) / kBlockK);
+  g.tiles_m = (int)((M + kTileM - 1) / kTileM);
+  g.tiles_n = (int)((N + kTileN - 1) / kTileN);
+  // Tiles rarely fill the last wave: cut the reduction in two where that wastes less of it (two parts added to
+  // zero give the same sum in either order; more parts would not).
+  const size_t tiles = (size_t)g.tiles_m * g.tiles_n, sms = (size_t)sm_count();
+  const size_t waves1 = 2 * ((tiles + sms - 1) / sms), waves2 = (2 * tiles + sms - 1) / sms;   // in half tiles
+  g.splits = waves2 < waves1 && g.k_blocks >= 16 ? 2 : 1;
+  if (g.splits > 1 && cudaMemsetAsync(d, 0, M * N * sizeof(float), st) != cudaSuccess)
+    return fail(SMORE_ERR_CUDA, "dot: cudaMemsetAsync failed");
+  if (int rc = allow_large_smem(split_gemm_kernel, kGemmSmem)) return rc;
+  const unsigned grid = (unsigned)std::min(tiles * g.splits, sms);
+  split_gemm_kernel<<<grid, kGemmThreads, kGemmSmem, st>>>(map_a, map_b, g);
+  return check_launch("split_gemm_kernel");
+}
+
+}  // namespace smore
+
+using namespace smore;
+
+extern "C" {
+
+int smore_split_status(int* status) {   // not part of the public header; smore_async_status adds it in
+  int v = 0;
+  if (cudaMemcpyFromSymbol(&v, g_split_status, sizeof(int)) != cudaSuccess)
+    return fail(SMORE_ERR_CUDA, "async_status: cannot read the status word");
+  *status = v;
+  return SMORE_OK;
+}
+
+int smore_split_status_clear(void) {
+  const int zero = 0;
+  if (cudaMemcpyToSymbol(g_split_status, &zero, sizeof(int)) != cudaSuccess)
+    return fail(SMORE_ERR_CUDA, "async_status_clear: cannot write the status word");
+  return SMORE_OK;
+}
+
+}  // extern "C"
