@@ -8,6 +8,8 @@
 //   fwd(e0, e1, q0, q1, acc[kNOut])                       adds one element's term(s)
 //   bwd(g[kNOut], e0, e1, q0, q1, ge0, ge1, gq0, gq1)     adds one element's gradients; q0 went through prep()
 //   kPositive / bwd_pos                                   a cheaper bwd for elements whose q1 is positive
+//   kFast / fwd_fast                                      a cheaper fwd for finite operands: acc[0] turns NaN where
+//                                                         fwd would not, and such a cell is taken again with fwd
 // Semantics, tie rules included, follow the reference functors
 // (smore/common/torchext/dist_kernel.h): sign(0) counts as -1 (:74,:97,:141), the box
 // "out" gradient flows when |e-c|-o is exactly 0 (:71), the box "in" test is strict (:94),
@@ -27,6 +29,8 @@ template <>
 __device__ __forceinline__ double t_abs<double>(double x) { return fabs(x); }
 __device__ __forceinline__ float t_min(float a, float b) { return fminf(a, b); }
 __device__ __forceinline__ double t_min(double a, double b) { return fmin(a, b); }
+__device__ __forceinline__ float t_max(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ double t_max(double a, double b) { return fmax(a, b); }
 __device__ __forceinline__ float t_sqrt_eps(float s) { return sqrtf(s + 1e-20f); }
 __device__ __forceinline__ double t_sqrt_eps(double s) { return sqrt(s + 1e-20); }
 __device__ __forceinline__ float t_rsqrt_eps(float s) { return rsqrtf(s + 1e-20f); }
@@ -40,6 +44,7 @@ __device__ __forceinline__ float t_xor_sign(float x, float y) {
 
 struct TermBase {
   static constexpr bool kPositive = false;
+  static constexpr bool kFast = false;
   template <typename T>
   __device__ __forceinline__ static T prep(T q0) { return q0; }
   template <typename T>
@@ -89,8 +94,16 @@ struct TermBoxBoth : TermBase {
   static constexpr int kId = SMORE_DIST_BOX_BOTH, kMul = 1, kNQ = 2, kNOut = 2;
   template <typename T>
   __device__ __forceinline__ static void fwd(T e0, T, T c, T o, T* acc) {
-    // max(a - o, 0) as a - min(a, o): the same value bit for bit (the difference of equal numbers is
-    // +0), and the minimum is needed anyway: five instructions per term instead of six
+    const T a = t_abs(e0 - c);
+    acc[0] += t_max(a - o, T(0));     // 0 for a NaN
+    acc[1] += t_abs(t_min(a, o));
+  }
+  // max(a - o, 0) as a - min(a, o): the same value bit for bit (the difference of equal numbers is +0), and
+  // the minimum is needed anyway: five instructions per term instead of six.  NaN for a NaN or for infinite a
+  // and o, where the term is 0; the sum of terms >= 0 is never NaN, so a NaN sum tells.
+  static constexpr bool kFast = true;
+  template <typename T>
+  __device__ __forceinline__ static void fwd_fast(T e0, T, T c, T o, T* acc) {
     const T a = t_abs(e0 - c);
     const T m = t_min(a, o);
     acc[0] += a - m;

@@ -78,6 +78,22 @@ __device__ __forceinline__ void copy_async(float* smem, const float* gmem, bool 
   else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(gmem), "r"(bytes) : "memory");
 }
 
+template <class Term>
+__device__ __forceinline__ void tile_term(float e0, float e1, float q0, float q1, float* acc) {
+  if constexpr (Term::kFast) Term::fwd_fast(e0, e1, q0, q1, acc);
+  else Term::fwd(e0, e1, q0, q1, acc);
+}
+
+// First output of one cell with Term::fwd, in the order of the dims as everywhere.
+template <class Term>
+__device__ __noinline__ float exact_cell(const SharedArgs& a, int b, long long row) {
+  const float* e = a.ent + (size_t)row * a.dim * Term::kMul;
+  const float *q0 = a.first + (size_t)b * a.dim, *q1 = Term::kNQ == 2 ? a.second + (size_t)b * a.dim : q0;
+  float acc[Term::kNOut] = {};
+  for (int d = 0; d < a.dim; ++d) Term::fwd(e[d], Term::kMul == 2 ? e[a.dim + d] : e[d], q0[d], q1[d], acc);
+  return acc[0];
+}
+
 // Scores of the tile (queries b0.., candidates k0..) into acc: thread (ty, tx) owns queries
 // b0 + ty + kTileTy * i and candidates k0 + tx + kTileTx * j.  Every cell accumulates its terms in the
 // order of the embedding dim, one after the other, so a (query, candidate) pair gets the same value
@@ -153,10 +169,10 @@ __device__ __forceinline__ void tile_scores(const SharedArgs& a, TileSmem<Term>&
       for (int i = 0; i < kCellsB; ++i)
 #pragma unroll
         for (int j = 0; j < kCellsK; ++j) {
-          Term::fwd(e0[j].x, e1[j].x, q0[i].x, q1[i].x, acc[i][j]);
-          Term::fwd(e0[j].y, e1[j].y, q0[i].y, q1[i].y, acc[i][j]);
-          Term::fwd(e0[j].z, e1[j].z, q0[i].z, q1[i].z, acc[i][j]);
-          Term::fwd(e0[j].w, e1[j].w, q0[i].w, q1[i].w, acc[i][j]);
+          tile_term<Term>(e0[j].x, e1[j].x, q0[i].x, q1[i].x, acc[i][j]);
+          tile_term<Term>(e0[j].y, e1[j].y, q0[i].y, q1[i].y, acc[i][j]);
+          tile_term<Term>(e0[j].z, e1[j].z, q0[i].z, q1[i].z, acc[i][j]);
+          tile_term<Term>(e0[j].w, e1[j].w, q0[i].w, q1[i].w, acc[i][j]);
         }
     }
     if (V == 1) {   // the up to three last dims of a row whose length is no multiple of four
@@ -168,10 +184,18 @@ __device__ __forceinline__ void tile_scores(const SharedArgs& a, TileSmem<Term>&
 #pragma unroll
           for (int j = 0; j < kCellsK; ++j) {
             const float e0 = st.e[0][tx + kTileTx * j][d];
-            Term::fwd(e0, Term::kMul == 2 ? st.e[Term::kMul - 1][tx + kTileTx * j][d] : e0, q0, q1, acc[i][j]);
+            tile_term<Term>(e0, Term::kMul == 2 ? st.e[Term::kMul - 1][tx + kTileTx * j][d] : e0, q0, q1, acc[i][j]);
           }
         }
     }
+  }
+  if constexpr (Term::kFast) {   // cells with NaN operands (or an infinite distance to an infinite box)
+#pragma unroll
+    for (int i = 0; i < kCellsB; ++i)
+#pragma unroll
+      for (int j = 0; j < kCellsK; ++j)
+        if (acc[i][j][0] != acc[i][j][0] && b0 + ty + kTileTy * i < a.B)
+          acc[i][j][0] = exact_cell<Term>(a, b0 + ty + kTileTy * i, max(sm.rows[tx + kTileTx * j], 0LL));
   }
 }
 
