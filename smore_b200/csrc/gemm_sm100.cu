@@ -17,6 +17,8 @@
 // points report SMORE_ERR_BAD_SHAPE and callers use the SIMT tile kernels.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "gemm_split.cuh"
 
@@ -148,6 +150,17 @@ static int run_tf32(const float* A, const float* B, float* D, int M, int N, int 
 
 using namespace smore;
 
+#ifdef SMORE_HAVE_CUTLASS
+// Candidates whose planes are held at a time: the planes of one such part (6 bytes per element of its rows, and
+// of its gradient block and that one's transpose) take at most 1.6 GB however long the list is.  A whole
+// entity table scored in one call would otherwise need one and a half times its size as scratch.  The
+// boundary is far above training lists (a list of 8192 is one part up to 2 B + W = 32768).
+static size_t candidates_per_part(size_t B, size_t K, size_t W) {
+  const size_t most = std::max<size_t>(256, ((size_t)1 << 28) / (2 * B + W) / 256 * 256);
+  return std::min(K, most);
+}
+#endif
+
 static int check_sizes(size_t B, size_t K, size_t W) {
   if (!B || !K || !W) return fail(SMORE_ERR_BAD_SHAPE, "dot: sizes must be positive");
   if (B > (1u << 30) || K > (1u << 30) || W > (1u << 30)) return fail(SMORE_ERR_TOO_LARGE, "dot: size too large");
@@ -176,8 +189,10 @@ size_t smore_dot_workspace_bytes(size_t B, size_t K, size_t W, int precision) {
 #ifdef SMORE_HAVE_CUTLASS
   if (check_sizes(B, K, W)) return 0;
   if (precision == SMORE_DOT_FP32) {
-    const size_t forward = split_plane_bytes(B, W) + split_plane_bytes(K, W);
-    const size_t backward = split_plane_bytes(B, K) + split_plane_bytes(K, B) + split_plane_bytes(W, K) + split_plane_bytes(W, B);
+    const size_t part = candidates_per_part(B, K, W);
+    const size_t forward = split_plane_bytes(B, W) + split_plane_bytes(part, W);
+    const size_t backward =
+        split_plane_bytes(B, part) + split_plane_bytes(part, B) + split_plane_bytes(W, part) + split_plane_bytes(W, B);
     return 1024 + (forward > backward ? forward : backward);
   }
   size_t n0 = 0, n1 = 0, n2 = 0;
@@ -230,11 +245,16 @@ int smore_dot_forward_shared(const float* cand, const float* query, float* dst, 
   cudaStream_t st = (cudaStream_t)stream;
   if (precision == SMORE_DOT_FP32) {
     if (!workspace || workspace_bytes < smore_dot_workspace_bytes(B, K, W, precision)) return gemm_status(kWorkspace, 0, 0, 0);
+    const size_t part = candidates_per_part(B, K, W);
     Planes ws(workspace);
-    void *q = ws.take(B, W), *c = ws.take(K, W);
-    if (int rc = split_planes(query, B, W, q, nullptr, st)) return rc;
-    if (int rc = split_planes(cand, K, W, c, nullptr, st)) return rc;
-    return split_gemm(q, c, dst, B, K, W, st);
+    void *q = ws.take(B, W), *c = ws.take(part, W);
+    if (int rc = split_planes(query, W, B, W, q, nullptr, st)) return rc;
+    for (size_t k = 0; k < K; k += part) {
+      const size_t n = std::min(part, K - k);
+      if (int rc = split_planes(cand + k * W, W, n, W, c, nullptr, st)) return rc;
+      if (int rc = split_gemm(q, c, dst + k, K, false, B, n, W, st)) return rc;
+    }
+    return SMORE_OK;
   }
   return run_tf32<RowM, ColM, kLayoutRowCol>(query, cand, dst, (int)B, (int)K, (int)W, workspace, workspace_bytes, st, nullptr);
 #else
@@ -254,13 +274,18 @@ int smore_dot_backward_shared(const float* gout, const float* cand, const float*
   // g_query[B, W] = gout[B, K] . cand[K, W];  g_cand[K, W] = gout^T[K, B] . query[B, W]
   if (precision == SMORE_DOT_FP32) {
     if (!workspace || workspace_bytes < smore_dot_workspace_bytes(B, K, W, precision)) return gemm_status(kWorkspace, 0, 0, 0);
+    const size_t part = candidates_per_part(B, K, W);
     Planes ws(workspace);
-    void *g = ws.take(B, K), *gt = ws.take(K, B), *ct = ws.take(W, K), *qt = ws.take(W, B);
-    if (int rc = split_planes(gout, B, K, g, gt, st)) return rc;
-    if (int rc = split_planes(cand, K, W, nullptr, ct, st)) return rc;
-    if (int rc = split_planes(query, B, W, nullptr, qt, st)) return rc;
-    if (int rc = split_gemm(g, ct, g_query, B, W, K, st)) return rc;
-    return split_gemm(gt, qt, g_cand, K, W, B, st);
+    void *g = ws.take(B, part), *gt = ws.take(part, B), *ct = ws.take(W, part), *qt = ws.take(W, B);
+    if (int rc = split_planes(query, W, B, W, nullptr, qt, st)) return rc;
+    for (size_t k = 0; k < K; k += part) {
+      const size_t n = std::min(part, K - k);
+      if (int rc = split_planes(gout + k, K, B, n, g, gt, st)) return rc;
+      if (int rc = split_planes(cand + k * W, W, n, W, nullptr, ct, st)) return rc;
+      if (int rc = split_gemm(g, ct, g_query, W, k > 0, B, W, n, st)) return rc;
+      if (int rc = split_gemm(gt, qt, g_cand + k * W, W, false, n, W, B, st)) return rc;
+    }
+    return SMORE_OK;
   }
   if (int rc = run_tf32<RowM, RowM, kLayoutRowRow>(gout, cand, g_query, (int)B, (int)W, (int)K, workspace, workspace_bytes, st,
                                                    nullptr))

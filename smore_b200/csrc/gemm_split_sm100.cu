@@ -45,19 +45,21 @@ __device__ __forceinline__ void split3(float x, __nv_bfloat16 (&p)[3]) {
   p[2] = __float2bfloat16_rn(r - __bfloat162float(p[1]));
 }
 
-// One 64 x 64 block per CTA.  plain: [3][rows][ld], transposed: [3][cols][ld_t]; either may be nullptr.
+// One 64 x 64 block per CTA, the blocks of a row of blocks next to each other.  plain: [3][rows][ld],
+// transposed: [3][cols][ld_t]; either may be nullptr.  x: [rows, cols], ld_x floats from row to row.
 __global__ void __launch_bounds__(256)
-    split_planes_kernel(const float* __restrict__ x, int rows, int cols, __nv_bfloat16* __restrict__ plain, size_t ld,
-                        __nv_bfloat16* __restrict__ transposed, size_t ld_t) {
+    split_planes_kernel(const float* __restrict__ x, size_t ld_x, int rows, int cols, __nv_bfloat16* __restrict__ plain,
+                        size_t ld, __nv_bfloat16* __restrict__ transposed, size_t ld_t) {
   __shared__ float tile[kSplitTile][kSplitTile + 1];
-  const int r0 = blockIdx.y * kSplitTile, c0 = blockIdx.x * kSplitTile;
+  const unsigned col_blocks = (unsigned)(cols + kSplitTile - 1) / kSplitTile;
+  const int r0 = (int)(blockIdx.x / col_blocks) * kSplitTile, c0 = (int)(blockIdx.x % col_blocks) * kSplitTile;
   const int t = threadIdx.x;
   {
     // 4 floats per thread and pass; cols is a multiple of 4
     const int c = c0 + (t & 15) * 4;
     for (int r = t >> 4; r < kSplitTile; r += 16) {
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (r0 + r < rows && c < cols) v = __ldg(reinterpret_cast<const float4*>(x + (size_t)(r0 + r) * cols + c));
+      if (r0 + r < rows && c < cols) v = __ldg(reinterpret_cast<const float4*>(x + (size_t)(r0 + r) * ld_x + c));
       float* d = &tile[r][(t & 15) * 4];
       d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
     }
@@ -101,9 +103,11 @@ constexpr int kGemmSmem = kStages * kStageBytes + 1024 /* alignment */;
 
 struct GemmArgs {
   float* d;              // [M, N] row-major
+  size_t ld_d;           // floats from row to row of d
   int M, N;
+  bool add;              // add to d
   int k_blocks;          // stages of the whole reduction
-  int splits;            // parts the reduction is cut into; > 1: parts are added into a zeroed d
+  int splits;            // parts the reduction is cut into; > 1: parts are added into d
   int tiles_m, tiles_n;
 };
 
@@ -316,12 +320,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       }
       const int m = it.m0 + quarter * 32 + lane, n0 = it.n0 + half * (kTileN / 2);
       if (ok && m < g.M && it.k_begin < it.k_end) {
-        float* out = g.d + (size_t)m * g.N + n0;
+        float* out = g.d + (size_t)m * g.ld_d + n0;
 #pragma unroll
         for (int c = 0; c < kTileN / 2; c += 4) {
           if (n0 + c >= g.N) continue;                // N is a multiple of 4
           const float4 v = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
-          if (g.splits > 1) atomicAdd(reinterpret_cast<float4*>(out + c), v);
+          if (g.add) atomicAdd(reinterpret_cast<float4*>(out + c), v);
           else *reinterpret_cast<float4*>(out + c) = v;
         }
       }
@@ -358,10 +362,12 @@ static EncodeTiled encode_tiled() {
 size_t split_pitch(size_t k) { return (k + 7) & ~(size_t)7; }
 size_t split_plane_bytes(size_t rows, size_t k) { return (3 * rows * split_pitch(k) * 2 + 1023) & ~(size_t)1023; }
 
-int split_planes(const float* x, size_t rows, size_t cols, void* plain, void* transposed, cudaStream_t st) {
-  const dim3 grid((unsigned)((cols + kSplitTile - 1) / kSplitTile), (unsigned)((rows + kSplitTile - 1) / kSplitTile));
-  split_planes_kernel<<<grid, 256, 0, st>>>(x, (int)rows, (int)cols, static_cast<__nv_bfloat16*>(plain), split_pitch(cols),
-                                            static_cast<__nv_bfloat16*>(transposed), split_pitch(rows));
+int split_planes(const float* x, size_t ld_x, size_t rows, size_t cols, void* plain, void* transposed, cudaStream_t st) {
+  const size_t blocks = ((cols + kSplitTile - 1) / kSplitTile) * ((rows + kSplitTile - 1) / kSplitTile);
+  if (blocks > 0x7fffffff) return fail(SMORE_ERR_TOO_LARGE, "dot: operand of %zu x %zu is too large", rows, cols);
+  split_planes_kernel<<<(unsigned)blocks, 256, 0, st>>>(x, ld_x, (int)rows, (int)cols, static_cast<__nv_bfloat16*>(plain),
+                                                        split_pitch(cols), static_cast<__nv_bfloat16*>(transposed),
+                                                        split_pitch(rows));
   return check_launch("split_planes_kernel");
 }
 
@@ -379,23 +385,26 @@ static int plane_map(CUtensorMap* map, const void* planes, size_t rows, size_t k
   return SMORE_OK;
 }
 
-int split_gemm(const void* a_planes, const void* b_planes, float* d, size_t M, size_t N, size_t K, cudaStream_t st) {
+int split_gemm(const void* a_planes, const void* b_planes, float* d, size_t ld_d, bool add, size_t M, size_t N, size_t K,
+               cudaStream_t st) {
   CUtensorMap map_a, map_b;
   if (int rc = plane_map(&map_a, a_planes, M, K, kTileM)) return rc;
   if (int rc = plane_map(&map_b, b_planes, N, K, kTileN)) return rc;
   GemmArgs g;
   g.d = d;
+  g.ld_d = ld_d;
   g.M = (int)M;
   g.N = (int)N;
   g.k_blocks = (int)((K + kBlockK - 1) / kBlockK);
   g.tiles_m = (int)((M + kTileM - 1) / kTileM);
   g.tiles_n = (int)((N + kTileN - 1) / kTileN);
   // Tiles rarely fill the last wave: cut the reduction in two where that wastes less of it (two parts added to
-  // zero give the same sum in either order; more parts would not).
+  // zero give the same sum in either order; more parts, or two added to something, would not).
   const size_t tiles = (size_t)g.tiles_m * g.tiles_n, sms = (size_t)sm_count();
   const size_t waves1 = 2 * ((tiles + sms - 1) / sms), waves2 = (2 * tiles + sms - 1) / sms;   // in half tiles
-  g.splits = waves2 < waves1 && g.k_blocks >= 16 ? 2 : 1;
-  if (g.splits > 1 && cudaMemsetAsync(d, 0, M * N * sizeof(float), st) != cudaSuccess)
+  g.splits = !add && waves2 < waves1 && g.k_blocks >= 16 ? 2 : 1;
+  g.add = add || g.splits > 1;
+  if (g.splits > 1 && cudaMemset2DAsync(d, ld_d * sizeof(float), 0, N * sizeof(float), M, st) != cudaSuccess)
     return fail(SMORE_ERR_CUDA, "dot: cudaMemsetAsync failed");
   if (int rc = allow_large_smem(split_gemm_kernel, kGemmSmem)) return rc;
   const unsigned grid = (unsigned)std::min(tiles * g.splits, sms);
