@@ -88,7 +88,7 @@ struct Lookup {
   std::string name;
   std::weak_ptr<StepPlan> plan;
   bool received = false;            // a gradient producer has run for this lookup
-  int n_consumers = 0;              // distance ops that took this lookup's rows in the forward pass
+  int n_consumers = 0;              // ops that took this lookup's rows in the forward pass
 };
 
 struct StepPlan {
@@ -297,6 +297,13 @@ bool needs_graph(std::initializer_list<const Tensor*> inputs) {
   return false;
 }
 
+// The nodes here have no forward-mode rule: refuse instead of dropping the tangent.
+void no_tangents(std::initializer_list<const Tensor*> inputs) {
+  for (const Tensor* t : inputs)
+    TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !t->_fw_grad(/*level=*/0).defined(),
+                                "forward-mode automatic differentiation is not supported by this op");
+}
+
 template <class N>
 void link(const std::shared_ptr<N>& node, std::initializer_list<const Tensor*> inputs, std::initializer_list<Tensor*> outputs) {
   torch::autograd::edge_list edges;
@@ -475,6 +482,8 @@ Tensor gather(const RowCore& core, const Tensor& idx) {
 Tensor dot_scores(const std::shared_ptr<RowCore>& core, const std::shared_ptr<Lookup>& lk, const Tensor& entity, const Tensor& first,
                   const Tensor& second, const QueryView& qv, int64_t K, int64_t W, int precision) {
   const Tensor& dev = core ? core->table : entity;
+  no_tangents({&entity, &first, &second});
+  if (core) lk->n_consumers += 1;
   c10::cuda::CUDAGuard guard(dev.device());
   Tensor cand, query, dst;
   {
@@ -521,6 +530,7 @@ py::object rows_dist(const std::shared_ptr<RowCore>& core, const std::shared_ptr
   if (core->width() != row_parts(dist_id) * qv.dim)
     throw py::value_error("table rows must be " + std::to_string(row_parts(dist_id)) + " x the query dim");
   check_broadcast(be, ne, qv.bc, qv.nc);
+  no_tangents({&first, &second});
   lk->n_consumers += 1;
   const int64_t bsize = std::max(be, qv.bc), num = std::max(ne, qv.nc);
   const bool both = dist_id == kBoxBoth;
@@ -629,6 +639,7 @@ py::object dense_dist(int dist_id, const Tensor& entity, const Tensor& first, co
   if (W != row_parts(dist_id) * qv.dim)
     throw py::value_error("entity rows must be " + std::to_string(row_parts(dist_id)) + " x the query dim");
   check_broadcast(be, ne, qv.bc, qv.nc);
+  no_tangents({&entity, &first, &second});
   const int64_t bsize = std::max(be, qv.bc), num = std::max(ne, qv.nc);
   c10::cuda::CUDAGuard guard(entity.device());
   Tensor e, q0, q1, d0, d1;
@@ -699,6 +710,7 @@ struct GatherNode : public Node {
 
 Tensor lookup_tensor(const std::shared_ptr<RowCore>& core, const std::shared_ptr<Lookup>& lk) {
   c10::cuda::CUDAGuard guard(core->table.device());
+  lk->n_consumers += 1;
   Tensor out;
   {
     at::AutoDispatchBelowADInplaceOrView below;
@@ -792,6 +804,8 @@ py::object path_embed(int geometry, const std::shared_ptr<RowCore>& core, const 
                       const std::optional<Tensor>& off_opt, const Tensor& rel_ids, bool relu_offset, double phase_scale) {
   const Tensor start = start_opt ? *start_opt : Tensor(), off = off_opt ? *off_opt : Tensor();
   const Tensor start_offset = start_offset_opt ? *start_offset_opt : Tensor();
+  no_tangents({&start, &start_offset, &rel, &off});
+  if (core) lk->n_consumers += 1;
   c10::cuda::CUDAGuard guard(rel.device());
   const bool two = geometry == kRotation || geometry == kComplexProduct;
   const bool has_off = geometry == kAdd && off.defined();
@@ -851,9 +865,14 @@ struct Answers {
   const int64_t* ids() const { return ptr() + 2 * (Q + 1); }
 };
 
-void append_ids(PyObject* list, int64_t limit, std::vector<int64_t>& out) {
-  py::object fast = py::reinterpret_steal<py::object>(PySequence_Fast(list, "answers must be iterables of candidate ids"));
+py::object as_list(PyObject* iterable) {   // itself where it is a list or tuple
+  py::object fast = py::reinterpret_steal<py::object>(PySequence_Fast(iterable, "answers must be iterables of candidate ids"));
   if (!fast) throw py::error_already_set();
+  return fast;
+}
+
+void append_ids(PyObject* list, int64_t limit, std::vector<int64_t>& out) {
+  const py::object fast = as_list(list);
   const Py_ssize_t n = PySequence_Fast_GET_SIZE(fast.ptr());
   PyObject** items = PySequence_Fast_ITEMS(fast.ptr());
   for (Py_ssize_t i = 0; i < n; ++i) {
@@ -861,6 +880,7 @@ void append_ids(PyObject* list, int64_t limit, std::vector<int64_t>& out) {
     if (PyLong_Check(items[i])) {
       v = PyLong_AsLongLong(items[i]);
     } else {
+      if (PyUnicode_Check(items[i]) || PyBytes_Check(items[i])) throw py::type_error("answer ids must be numbers");
       py::object num = py::reinterpret_steal<py::object>(PyNumber_Long(items[i]));
       if (!num) throw py::error_already_set();
       v = PyLong_AsLongLong(num.ptr());
@@ -871,16 +891,19 @@ void append_ids(PyObject* list, int64_t limit, std::vector<int64_t>& out) {
   }
 }
 
-Answers pack_answers(const py::sequence& easy, const py::sequence& hard, int64_t Q, int64_t n_candidates, const Tensor& like) {
-  if ((int64_t)py::len(easy) != Q || (int64_t)py::len(hard) != Q)
+Answers pack_answers(const py::object& easy_lists, const py::object& hard_lists, int64_t Q, int64_t n_candidates, const Tensor& like) {
+  if ((int64_t)py::len(easy_lists) != Q || (int64_t)py::len(hard_lists) != Q)
+    throw py::value_error("one easy and one hard answer list per query");
+  const py::object easy = as_list(easy_lists.ptr()), hard = as_list(hard_lists.ptr());
+  if (PySequence_Fast_GET_SIZE(easy.ptr()) != Q || PySequence_Fast_GET_SIZE(hard.ptr()) != Q)
     throw py::value_error("one easy and one hard answer list per query");
   Answers a;
   a.Q = Q;
   std::vector<int64_t> ids, ptr{0}, hard_ptr{0};
   for (int64_t q = 0; q < Q; ++q) {
-    append_ids(py::object(easy[q]).ptr(), n_candidates, ids);
+    append_ids(PySequence_Fast_GET_ITEM(easy.ptr(), q), n_candidates, ids);
     const int64_t easy_end = (int64_t)ids.size();
-    append_ids(py::object(hard[q]).ptr(), n_candidates, ids);
+    append_ids(PySequence_Fast_GET_ITEM(hard.ptr(), q), n_candidates, ids);
     a.hard_counts.push_back((int64_t)ids.size() - easy_end);
     a.longest = std::max(a.longest, (int64_t)ids.size() - ptr.back());
     ptr.push_back((int64_t)ids.size());
@@ -908,7 +931,7 @@ py::list split_ranks(const Tensor& ranks, const Answers& a) {
   return out;
 }
 
-py::list filtered_ranks(Tensor logits, const py::sequence& easy, const py::sequence& hard) {
+py::list filtered_ranks(Tensor logits, const py::object& easy, const py::object& hard) {
   if (logits.dim() != 2 || logits.scalar_type() != at::kFloat || !logits.is_cuda())
     throw py::type_error("logits must be a 2-D float32 CUDA tensor");
   const int64_t Q = logits.size(0), N = logits.size(1);
@@ -928,7 +951,7 @@ py::list filtered_ranks(Tensor logits, const py::sequence& easy, const py::seque
 }
 
 py::list score_and_rank(int dist_id, const Tensor& table, const Tensor& first, const std::optional<Tensor>& second_opt,
-                        const py::sequence& easy, const py::sequence& hard, double gamma, double cen) {
+                        const py::object& easy, const py::object& hard, double gamma, double cen) {
   if (table.scalar_type() != at::kFloat || !table.is_cuda() || !table.is_contiguous())
     throw py::type_error("table must be a contiguous float32 CUDA tensor");
   c10::cuda::CUDAGuard guard(table.device());

@@ -240,9 +240,7 @@ class EmbeddingOptimizer(object):
     # ---- construction --------------------------------------------------------------------------
     def __init__(self, args, sp_embed, gpu_id, lazy_names=None):
         self.args = args
-        # the module holds this object (fwd_delegate below); holding it back strongly would leave the table
-        # and its state to the cycle collector.  With share_optim_stats the state lives on the module.
-        self._sparse_embed = weakref.ref(sp_embed) if not getattr(args, "share_optim_stats", False) else (lambda: sp_embed)
+        self._sparse_embed = self._reference_to(sp_embed)
         self.gpu_id = gpu_id
         if not sp_embed.embedding.is_cuda:
             raise _lib.SmoreError("the embedding table must be in GPU memory (move the module to cuda:%s first)"
@@ -268,8 +266,7 @@ class EmbeddingOptimizer(object):
             lazy_names = tuple(x for x in env.split(",") if x)
         self.lazy_names = tuple(lazy_names)
         self._local_state = {}
-        self.core = _lib.host().RowCore(self.table, self.dummy_tensor, _lib.OPT_IDS[self.opt_name], self.squeeze,
-                                        self.opt_name == "adam" and not self.share_optim_stats)
+        self.core = self._new_core()
         if self.share_optim_stats:
             for name in self.state_names:
                 if not hasattr(sp_embed, name):
@@ -278,6 +275,39 @@ class EmbeddingOptimizer(object):
         else:
             self.prepare_embed(args, optim_mode, sp_embed, self._register_local)
         self.zero_grad()
+
+    def __getstate__(self):
+        """Copies and pickles between two steps: the native core goes as its counters."""
+        state = dict(self.__dict__)
+        if "_sparse_embed" in state:
+            state["_sparse_embed"] = self._sparse_embed()
+        core = state.pop("core", None)
+        if core is not None:
+            state["_counters"] = (core.step, None if core.step_dev is None else int(core.step_dev))
+        return state
+
+    def __setstate__(self, state):
+        counters = state.pop("_counters", None)
+        self.__dict__.update(state)
+        if "_sparse_embed" in state:
+            self._sparse_embed = self._reference_to(state["_sparse_embed"])
+        if counters is not None:
+            step, step_dev = counters
+            self.core = self._new_core()
+            if step_dev is not None:
+                self.core.step = step_dev
+                self.core.use_device_step()
+            self.core.step = step
+
+    def _reference_to(self, embed):
+        # the module holds this object (fwd_delegate); holding it back strongly would leave the table
+        # and its state to the cycle collector.  With share_optim_stats the state lives on the module.
+        return weakref.ref(embed) if embed is not None and not getattr(self.args, "share_optim_stats", False) \
+            else (lambda: embed)
+
+    def _new_core(self):
+        return _lib.host().RowCore(self.table, self.dummy_tensor, _lib.OPT_IDS[self.opt_name], self.squeeze,
+                                   self.opt_name == "adam" and not self.share_optim_stats)
 
     def _register_local(self, name, tensor):
         self._local_state[name] = tensor.to(self.table.device)
