@@ -432,8 +432,8 @@ __global__ void __launch_bounds__(128)
                          float* __restrict__ logits) {
   __shared__ __align__(16) float q[2][kAnswerDims];
   __shared__ __align__(16) float e[kAnswersPerCta][Term::kMul][kAnswerDims + 4];
-  const int b = blockIdx.x;
-  const long long begin = answer_ptr[b] + (long long)blockIdx.y * kAnswersPerCta;
+  const int b = (int)(blockIdx.x % a.B);
+  const long long begin = answer_ptr[b] + (long long)(blockIdx.x / a.B) * kAnswersPerCta;
   const int n = (int)max(0LL, min((long long)kAnswersPerCta, answer_ptr[b + 1] - begin));
   if (n == 0) return;
   float acc[Term::kNOut];
@@ -671,13 +671,14 @@ static int score_filtered_ranks_impl(int dist_id, const float* table, size_t n_c
   cudaStream_t st = (cudaStream_t)stream;
   SharedArgs a_ans{table, answer_ids, first, second, (int)n_queries, (int)n_answers, (int)dim, (long long)n_candidates, 0, 0};
   SharedArgs a_all{table, nullptr, first, second, (int)n_queries, (int)n_candidates, (int)dim, 0, 0, 0};
-  const dim3 grid_ans((unsigned)n_queries, (unsigned)((max_answers + kAnswersPerCta - 1) / kAnswersPerCta));
+  const size_t grid_ans = n_queries * ((max_answers + kAnswersPerCta - 1) / kAnswersPerCta);
+  if (grid_ans > (size_t)INT_MAX) return fail(SMORE_ERR_TOO_LARGE, "score_filtered_ranks: too many answers");
   const size_t q_tiles = (n_queries + kTileB - 1) / kTileB, k_tiles = (n_candidates + kTileK - 1) / kTileK;
   // answers of a query tile kept on the SM: four CTAs per SM leave room for about a thousand (12 bytes each)
   const int cap = 1024;
 #define SCORE_RANK(TERM)                                                                                             \
   {                                                                                                                  \
-    answer_logits_kernel<TERM><<<grid_ans, 128, 0, st>>>(a_ans, answer_ptr, kind, (float)gamma, (float)cen, logits); \
+    answer_logits_kernel<TERM><<<(unsigned)grid_ans, 128, 0, st>>>(a_ans, answer_ptr, kind, (float)gamma, (float)cen, logits); \
     count_launches(1);                                                                                               \
     if (int rc = rank_sort_answers(logits, n_answers, answer_ptr, answer_ids, true, n_queries, n_answers,            \
                                    max_answers, w, st))                                                              \
