@@ -400,36 +400,36 @@ __global__ void __launch_bounds__(256)
 
 // UpdateArgs, adam_elem, adam_elem_rowwise: update_math.cuh
 
-// Adam for rows of at most 32 * NCH 16-byte chunks: every load of a row (gradient, parameters,
-// first moment and, with a full second moment, that too) is issued before anything is computed,
-// so each warp keeps 3-4 x NCH 512-byte requests in flight; the gradient is read once even when
-// the row-wise mean of its square is needed first.
-template <int NCH, bool ROWWISE>
+// Entries a warp takes at a time: one read of their row ids, then the rows one after the other (small batches keep
+// the warps' loads even).  Entries with a negative id were updated inside the backward pass
+// (smore_rows_backward_fused_adam) and cost nothing beyond that read.
+constexpr int kUpdateBatch = 8;
+__device__ __forceinline__ long long batch_row(const UpdateArgs& a, size_t batch, size_t nu, int lane) {
+  const size_t u = batch * kUpdateBatch + lane;
+  return lane < kUpdateBatch && u < nu ? a.uniq[u] : -1;
+}
+
+// Adam with a row-wise second moment for rows of at most 32 * NCH 16-byte chunks: every load of a row (gradient,
+// parameters, first moment) is issued before anything is computed, so each warp keeps 3 x NCH 512-byte requests
+// in flight; the gradient is read once although the mean of its square is needed first.
+template <int NCH>
 __global__ void __launch_bounds__(256) adam_rows_reg_kernel(UpdateArgs a) {
   load_dyn(a);
   const int lane = threadIdx.x & 31;
   const size_t nu = (size_t)max(a.n_unique[0], 0);
-  const size_t warps = (size_t)gridDim.x * (blockDim.x >> 5);
+  const size_t warps = (size_t)gridDim.x * (blockDim.x >> 5), batches = (nu + kUpdateBatch - 1) / kUpdateBatch;
   const int w4 = (int)(a.width >> 2);
-  // a warp takes kBatch consecutive entries of the list at a time: one read of their row ids, then the
-  // rows one after the other (small batches keep the warps' loads even).  Entries with a negative id
-  // were updated inside the backward pass (smore_rows_backward_fused_adam) and cost nothing here
-  // beyond that read.
-  constexpr int kBatch = 8;
-  for (size_t u0 = ((size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kBatch; u0 < nu;
-       u0 += warps * kBatch) {
-    const long long my_row = (lane < kBatch && u0 + lane < nu) ? a.uniq[u0 + lane] : -1;
+  for (size_t batch = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); batch < batches; batch += warps) {
+    const long long my_row = batch_row(a, batch, nu, lane);
     unsigned live = __ballot_sync(0xffffffffu, my_row >= 0);
     while (live) {
       const int l = __ffs(live) - 1;
       live &= live - 1;
       const long long row = __shfl_sync(0xffffffffu, my_row, l);
-      const size_t u = u0 + l;
-      const float4* g4 = reinterpret_cast<const float4*>(a.g_rows + u * a.width);
+      const float4* g4 = reinterpret_cast<const float4*>(a.g_rows + (batch * kUpdateBatch + l) * a.width);
       float4* p4 = reinterpret_cast<float4*>(a.table + (size_t)row * a.width);
       float4* m4 = reinterpret_cast<float4*>(a.m + (size_t)row * a.width);
-      float4* v4 = ROWWISE ? nullptr : reinterpret_cast<float4*>(a.v + (size_t)row * a.width);
-      float4 g[NCH], p[NCH], m[NCH], v[NCH];
+      float4 g[NCH], p[NCH], m[NCH];
 #pragma unroll
       for (int j = 0; j < NCH; ++j) {
         const int d = lane + 32 * j;
@@ -437,42 +437,82 @@ __global__ void __launch_bounds__(256) adam_rows_reg_kernel(UpdateArgs a) {
           g[j] = __ldcs(g4 + d);
           p[j] = p4[d];
           m[j] = m4[d];
-          if (!ROWWISE) v[j] = v4[d];
         }
       }
-      RowDenom denom = {1.f, 1.f};
-      float v_old = 0.f, v_new = 0.f;
-      if (ROWWISE) {
-        v_old = a.v[row];
-        float s = 0.f;
+      const float v_old = a.v[row];
+      float s = 0.f;
 #pragma unroll
-        for (int j = 0; j < NCH; ++j)
-          if (lane + 32 * j < w4) s += g[j].x * g[j].x + g[j].y * g[j].y + g[j].z * g[j].z + g[j].w * g[j].w;
-        const float g2mean = warp_sum(s) / (float)a.width;
-        v_new = v_old * a.beta2 + g2mean * a.omb2;
-        denom = rowwise_denom(v_new, a);
-      }
+      for (int j = 0; j < NCH; ++j)
+        if (lane + 32 * j < w4) s += g[j].x * g[j].x + g[j].y * g[j].y + g[j].z * g[j].z + g[j].w * g[j].w;
+      const float g2mean = warp_sum(s) / (float)a.width;
+      const float v_new = v_old * a.beta2 + g2mean * a.omb2;
+      const RowDenom denom = rowwise_denom(v_new, a);
 #pragma unroll
       for (int j = 0; j < NCH; ++j) {
         const int d = lane + 32 * j;
         if (d < w4) {
-          if (ROWWISE) {
-            adam_elem_rowwise(g[j].x, p[j].x, m[j].x, denom, a);
-            adam_elem_rowwise(g[j].y, p[j].y, m[j].y, denom, a);
-            adam_elem_rowwise(g[j].z, p[j].z, m[j].z, denom, a);
-            adam_elem_rowwise(g[j].w, p[j].w, m[j].w, denom, a);
-          } else {
-            adam_elem(g[j].x, p[j].x, m[j].x, v[j].x, a);
-            adam_elem(g[j].y, p[j].y, m[j].y, v[j].y, a);
-            adam_elem(g[j].z, p[j].z, m[j].z, v[j].z, a);
-            adam_elem(g[j].w, p[j].w, m[j].w, v[j].w, a);
-            v4[d] = v[j];
-          }
+          adam_elem_rowwise(g[j].x, p[j].x, m[j].x, denom, a);
+          adam_elem_rowwise(g[j].y, p[j].y, m[j].y, denom, a);
+          adam_elem_rowwise(g[j].z, p[j].z, m[j].z, denom, a);
+          adam_elem_rowwise(g[j].w, p[j].w, m[j].w, denom, a);
           p4[d] = p[j];
           m4[d] = m[j];
         }
       }
-      if (ROWWISE && lane == 0) a.v[row] = v_old + (v_new - v_old);
+      if (lane == 0) a.v[row] = v_old + (v_new - v_old);
+    }
+  }
+}
+
+// Adam with a full second moment: nothing is summed over a row, so a warp takes kUpdateBatch entries' piece of
+// 32 * C chunks and long rows are spread over several warps.  (One warp per row of 1000 floats held it in 128
+// registers, which left 8 warps on an SM, each waiting for its own loads and then for its own divisions:
+// 1136 us for RotatE's 168k rows with several contributors, 825 us like this, 4.7 GB; 8192 + 4096 rows of 1000
+// floats 96 -> 67 us.)
+template <int C>
+__global__ void __launch_bounds__(256) adam_full_kernel(UpdateArgs a, unsigned pieces) {
+  load_dyn(a);
+  const int lane = threadIdx.x & 31;
+  const size_t nu = (size_t)max(a.n_unique[0], 0);
+  const size_t warps = (size_t)gridDim.x * (blockDim.x >> 5);
+  const size_t items = (nu + kUpdateBatch - 1) / kUpdateBatch * pieces;
+  const size_t w4 = a.width >> 2;
+  for (size_t item = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); item < items; item += warps) {
+    const size_t batch = item / pieces;
+    const size_t d0 = (item - batch * pieces) * (32 * C) + lane;
+    const long long my_row = batch_row(a, batch, nu, lane);
+    unsigned live = __ballot_sync(0xffffffffu, my_row >= 0);
+    while (live) {
+      const int l = __ffs(live) - 1;
+      live &= live - 1;
+      const size_t row = (size_t)__shfl_sync(0xffffffffu, my_row, l) * w4;
+      const float4* g4 = reinterpret_cast<const float4*>(a.g_rows) + (batch * kUpdateBatch + l) * w4;
+      float4 *p4 = reinterpret_cast<float4*>(a.table) + row, *m4 = reinterpret_cast<float4*>(a.m) + row,
+             *v4 = reinterpret_cast<float4*>(a.v) + row;
+      float4 g[C], p[C], m[C], v[C];
+#pragma unroll
+      for (int j = 0; j < C; ++j) {
+        const size_t d = d0 + 32 * j;
+        if (d < w4) {
+          g[j] = __ldcs(g4 + d);
+          p[j] = p4[d];
+          m[j] = m4[d];
+          v[j] = v4[d];
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < C; ++j) {
+        const size_t d = d0 + 32 * j;
+        if (d < w4) {
+          adam_elem(g[j].x, p[j].x, m[j].x, v[j].x, a);
+          adam_elem(g[j].y, p[j].y, m[j].y, v[j].y, a);
+          adam_elem(g[j].z, p[j].z, m[j].z, v[j].z, a);
+          adam_elem(g[j].w, p[j].w, m[j].w, v[j].w, a);
+          v4[d] = v[j];
+          p4[d] = p[j];
+          m4[d] = m[j];
+        }
+      }
     }
   }
 }
@@ -858,16 +898,22 @@ static int update_rows_impl(int opt_id, float* table, float* m, float* v, const 
                    (!v || squeeze || aligned16(v));
   const int grid = warp_grid(capacity);
   const size_t w4 = width >> 2;
+  if (opt_id == SMORE_OPT_ADAM && vec && !a.squeeze) {
+    if (w4 <= 32) {
+      adam_full_kernel<1><<<grid, 256, 0, st>>>(a, 1u);
+    } else {
+      const size_t pieces = (w4 + 63) / 64;
+      if (pieces > (size_t)UINT32_MAX) return fail(SMORE_ERR_TOO_LARGE, "sparse_update_rows: width is too large");
+      adam_full_kernel<2><<<warp_grid(capacity * pieces), 256, 0, st>>>(a, (unsigned)pieces);
+    }
+    return check_launch("adam_full_kernel");
+  }
   if (opt_id == SMORE_OPT_ADAM && vec && w4 <= 256) {
     // rows of up to 1024 floats: the register-resident kernel
-#define ADAM_REG(NCH)                                                         \
-  if (a.squeeze) adam_rows_reg_kernel<NCH, true><<<grid, 256, 0, st>>>(a);    \
-  else adam_rows_reg_kernel<NCH, false><<<grid, 256, 0, st>>>(a)
-    if (w4 <= 32) { ADAM_REG(1); }
-    else if (w4 <= 64) { ADAM_REG(2); }
-    else if (w4 <= 128) { ADAM_REG(4); }
-    else { ADAM_REG(8); }
-#undef ADAM_REG
+    if (w4 <= 32) adam_rows_reg_kernel<1><<<grid, 256, 0, st>>>(a);
+    else if (w4 <= 64) adam_rows_reg_kernel<2><<<grid, 256, 0, st>>>(a);
+    else if (w4 <= 128) adam_rows_reg_kernel<4><<<grid, 256, 0, st>>>(a);
+    else adam_rows_reg_kernel<8><<<grid, 256, 0, st>>>(a);
     return check_launch("adam_rows_reg_kernel");
   }
 #define LAUNCH(OPT)                                                                  \

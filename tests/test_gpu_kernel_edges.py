@@ -259,6 +259,38 @@ def test_row_moment_update_divides_exactly(dim):
     assert same.all(), (np.argwhere(~same)[:5], got[~same][:5], want[~same][:5])
 
 
+@pytest.mark.parametrize("dim", [4, 128, 132, 256, 260, 1000, 1028])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 3000])
+def test_full_moment_update_in_pieces(dim, n):
+    """Rows of one piece, of several and with a last piece that is not full; batches that are not full;
+    entries whose update is done already (negative ids).  Against float64: a handful of roundings each."""
+    from smore_b200 import _lib
+    rows = 4 * n
+    g = torch.Generator(device="cuda").manual_seed(dim + n)
+    table = torch.randn(rows, dim, device="cuda", generator=g)
+    m, v = torch.randn(rows, dim, device="cuda", generator=g) * 1e-3, torch.rand(rows, dim, device="cuda", generator=g) * 1e-6
+    grad = torch.randn(n, dim, device="cuda", generator=g) * 1e-3
+    ids = torch.sort(torch.randperm(rows, device="cuda", generator=g)[:n])[0]
+    done = torch.rand(n, device="cuda", generator=g) < 0.3
+    before = [t.clone() for t in (table, m, v)]
+    listed = torch.where(done, ~ids, ids)
+    count = torch.tensor([n, 0], dtype=torch.int32, device="cuda")
+    _lib.check(_lib.lib().smore_sparse_update_rows(
+        _lib.OPT_IDS["adam"], table.data_ptr(), m.data_ptr(), v.data_ptr(), listed.data_ptr(), grad.data_ptr(), count.data_ptr(),
+        n, dim, 1e-2, 0.9, 0.999, 1e-8, 3, 0, torch.cuda.current_stream().cuda_stream), "update")
+    p64, m64, v64 = [t.double() for t in before]
+    r, gr = ids[~done], grad[~done].double()
+    m64[r] = 0.9 * m64[r] + 0.1 * gr
+    v64[r] = 0.999 * v64[r] + 0.001 * gr * gr
+    p64[r] -= 1e-2 / (1 - 0.9 ** 3) * m64[r] / ((v64[r] / (1 - 0.999 ** 3)).sqrt() + 1e-8)
+    for got, want in zip((table, m, v), (p64, m64, v64)):
+        close(got.cpu().numpy(), want.cpu().numpy(), RTOL)
+    for got, old in zip((table, m, v), before):
+        keep = torch.ones(rows, dtype=torch.bool, device="cuda")
+        keep[r] = False
+        assert torch.equal(got[keep], old[keep])
+
+
 # ---- evaluation ------------------------------------------------------------------------------------
 
 @pytest.mark.parametrize("Q,N", [(1, 63), (31, 64), (32, 65), (33, 4096), (64, 129), (70, 1000)])
@@ -291,6 +323,36 @@ def test_answers_that_are_no_ids_are_refused():
     for bad, error in (([8], ValueError), ([-1], ValueError), (["3"], TypeError), (3, TypeError)):
         with pytest.raises(error):
             ranking.filtered_ranks(logits, [[]], [bad])
+
+
+# ---- negative sampling -----------------------------------------------------------------------------
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("Q,k,per_query", [(1, 1, 0), (3, 5, 2), (1, 700, 9), (64, 33, 30), (2, 257, 1500), (40, 9000, 3),
+                                           (700, 1024, 31)])
+def test_draws_do_not_depend_on_the_launch(weighted, Q, k, per_query):
+    """One, two and four positions per thread, CTAs that span several queries, answers that fit on the SM and
+    that do not: every position draws what its counter gives, from packed tables as from three arrays."""
+    from smore_b200 import _lib, sampler
+    n = 5000
+    rng = np.random.default_rng(Q + k)
+    weights = rng.random(n) ** 4 + 1e-3 if weighted else None
+    csr = sampler.answers_csr([rng.choice(n, per_query, replace=False) for _ in range(Q)], "cuda")
+    s = sampler.NegativeSampler(n, "cuda", weights=weights, seed=11)
+    s.offset = 5
+    got = s.sample(Q, k, csr)
+    stream = torch.cuda.current_stream().cuda_stream
+    t = [None] * 3 if s.tables is None else [x.data_ptr() for x in s.tables]
+    one = torch.empty_like(got)
+    for q in (range(Q) if Q <= 64 else (0, 1, Q // 2, Q - 1)):       # a query by itself, from the arrays
+        a, b = int(csr[0][q]), int(csr[0][q + 1])
+        ptr = torch.tensor([0, b - a], device="cuda")
+        ids = csr[1][a:max(b, a + 1)]
+        for at in range(0, k, 300):                                   # and in pieces
+            m = min(300, k - at)
+            _lib.check(_lib.lib().smore_sample_negatives(11, 5 + q * k + at, n, *t, ptr.data_ptr(), ids.data_ptr(), 1, m,
+                                                         one[q, at:].data_ptr(), stream), "sample")
+        assert torch.equal(got[q], one[q]) and not torch.isin(got[q], csr[1][a:b]).any()
 
 
 # ---- the native host side --------------------------------------------------------------------------
