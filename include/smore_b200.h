@@ -454,6 +454,8 @@ SMORE_API int smore_score_hard_ranks(int dist_id, const float* table, size_t n_c
  * [n_queries + 1] / answer_ids: per query its answers in ascending order (CSR, device), or both NULL;
  * a draw that is an answer is repeated (at most 64 times).  Advance `offset` by n_queries * k per
  * call to continue the stream.
+ * smore_sample_negatives_packed: the same draws from tables of n_entities < 2^32 choices laid out as 16-byte
+ * entries {double prob_small; uint32_t choice_small, choice_large}, 16-byte aligned.
  * smore_negative_mask: is_negative[b, j] = 0.0 if negatives[j] is an answer of query b, else 1.0.
  * ------------------------------------------------------------------------------------------ */
 SMORE_API int smore_alias_build(const double* weights, size_t n, double* prob_small, int64_t* choice_small,
@@ -462,6 +464,9 @@ SMORE_API int smore_sample_negatives(uint64_t seed, uint64_t offset, size_t n_en
                            const int64_t* choice_small, const int64_t* choice_large,
                            const int64_t* answer_ptr, const int64_t* answer_ids, size_t n_queries, size_t k,
                            int64_t* negatives, void* stream);
+SMORE_API int smore_sample_negatives_packed(uint64_t seed, uint64_t offset, size_t n_entities, const void* entries,
+                                  const int64_t* answer_ptr, const int64_t* answer_ids, size_t n_queries, size_t k,
+                                  int64_t* negatives, void* stream);
 SMORE_API int smore_negative_mask(const int64_t* negatives, size_t k, const int64_t* answer_ptr,
                         const int64_t* answer_ids, size_t n_queries, float* is_negative, void* stream);
 

@@ -67,6 +67,7 @@ SIGNATURES = {
     "smore_hard_ranks": (_int, [_p, _sz, _sz, _p, _p, _sz, _sz, _p, _p, _p, _sz, _p]),
     "smore_score_hard_ranks": (_int, [_int, _p, _sz, _p, _p, _sz, _sz, _dbl, _dbl, _p, _p, _sz, _sz, _p, _p, _p, _sz, _p]),
     "smore_alias_build": (_int, [_p, _sz, _p, _p, _p]),
+    "smore_sample_negatives_packed": (_int, [ctypes.c_uint64, ctypes.c_uint64, _sz, _p, _p, _p, _sz, _sz, _p, _p]),
     "smore_sample_negatives": (_int, [ctypes.c_uint64, ctypes.c_uint64, _sz, _p, _p, _p, _p, _p, _sz, _sz, _p, _p]),
     "smore_negative_mask": (_int, [_p, _sz, _p, _p, _sz, _p, _p]),
     "smore_dot_available": (_int, []),

@@ -972,6 +972,25 @@ py::list score_and_rank(int dist_id, const Tensor& table, const Tensor& first, c
   return split_ranks(ranks, a);
 }
 
+// ---- negative sampling -------------------------------------------------------------------------------
+// Draws of smore_b200.sampler.NegativeSampler: `entries` the packed alias tables, or nothing for uniform draws.
+Tensor sample_negatives(uint64_t seed, uint64_t offset, int64_t n_entities, const std::optional<Tensor>& entries,
+                        const std::optional<Tensor>& answer_ptr, const std::optional<Tensor>& answer_ids, int64_t n_queries,
+                        int64_t k, const at::Device& device) {
+  c10::cuda::CUDAGuard guard(device);
+  Tensor out = at::empty({n_queries, k}, at::TensorOptions().dtype(at::kLong).device(guard.current_device()));
+  auto ids = [](const std::optional<Tensor>& t) { return t ? (const int64_t*)t->data_ptr() : nullptr; };
+  if (entries)
+    check(smore_sample_negatives_packed(seed, offset, n_entities, entries->data_ptr(), ids(answer_ptr), ids(answer_ids), n_queries,
+                                        k, (int64_t*)out.data_ptr(), stream_of(out)),
+          "smore_sample_negatives_packed");
+  else
+    check(smore_sample_negatives(seed, offset, n_entities, nullptr, nullptr, nullptr, ids(answer_ptr), ids(answer_ids), n_queries, k,
+                                 (int64_t*)out.data_ptr(), stream_of(out)),
+          "smore_sample_negatives");
+  return out;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_host, mod) {
@@ -1090,4 +1109,5 @@ PYBIND11_MODULE(_host, mod) {
   mod.def("path_embed", &path_embed);
   mod.def("filtered_ranks", &filtered_ranks);
   mod.def("score_and_rank", &score_and_rank);
+  mod.def("sample_negatives", &sample_negatives);
 }

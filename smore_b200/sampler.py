@@ -13,6 +13,9 @@ import torch
 from . import _lib
 
 
+_U64 = (1 << 64) - 1      # as ctypes takes an unsigned argument: modulo 2^64
+
+
 def build_alias_table(weights):
     """(prob_small float64 [n], choice_small int64 [n], choice_large int64 [n]) for non-negative
     weights, by the reference's procedure (alias_method.cpp:55-99); numpy arrays on the host."""
@@ -42,23 +45,32 @@ class NegativeSampler(object):
 
     def __init__(self, n_entities, device, weights=None, seed=0):
         self.n_entities, self.device, self.seed, self.offset = int(n_entities), torch.device(device), int(seed), 0
-        self.tables = None
+        self.tables = self._entries = None
         if weights is not None:
             if len(weights) != self.n_entities:
                 raise ValueError("one weight per entity")
             prob, small, large = build_alias_table(weights)
             self.tables = (torch.from_numpy(prob).to(self.device), torch.from_numpy(small).to(self.device),
                            torch.from_numpy(large).to(self.device))
+            if self.n_entities < 1 << 32:      # the same tables, one 16-byte entry per slot
+                entries = np.empty((self.n_entities, 2), np.int64)
+                entries[:, 0] = prob.view(np.int64)
+                entries[:, 1] = small | large << 32
+                self._entries = torch.from_numpy(entries).to(self.device)
 
     def _draw(self, n_queries, k, csr):
-        out = torch.empty(n_queries, k, dtype=torch.int64, device=self.device)
-        t = self.tables
-        with torch.cuda.device(self.device):
-            _lib.check(_lib.lib().smore_sample_negatives(
-                self.seed, self.offset, self.n_entities, None if t is None else t[0].data_ptr(),
-                None if t is None else t[1].data_ptr(), None if t is None else t[2].data_ptr(),
-                None if csr is None else csr[0].data_ptr(), None if csr is None else csr[1].data_ptr(), n_queries, k,
-                out.data_ptr(), torch.cuda.current_stream(self.device).cuda_stream), "smore_sample_negatives")
+        csr = csr if csr is not None else (None, None)
+        if self._entries is not None or self.tables is None:
+            out = _lib.host().sample_negatives(self.seed & _U64, self.offset & _U64, self.n_entities, self._entries, csr[0],
+                                               csr[1], n_queries, k, self.device)
+        else:
+            out = torch.empty(n_queries, k, dtype=torch.int64, device=self.device)
+            ptr = lambda t: None if t is None else t.data_ptr()
+            with torch.cuda.device(self.device):
+                _lib.check(_lib.lib().smore_sample_negatives(
+                    self.seed, self.offset, self.n_entities, *[t.data_ptr() for t in self.tables], ptr(csr[0]), ptr(csr[1]),
+                    n_queries, k, out.data_ptr(), torch.cuda.current_stream(self.device).cuda_stream),
+                    "smore_sample_negatives")
         self.offset += n_queries * k
         return out
 
