@@ -190,10 +190,15 @@ size_t smore_dot_workspace_bytes(size_t B, size_t K, size_t W, int precision) {
   if (check_sizes(B, K, W)) return 0;
   if (precision == SMORE_DOT_FP32) {
     const size_t part = candidates_per_part(B, K, W);
+    // (the last part of a list may be short, and be cut differently)
+    const size_t tail = K % part ? K % part : part;
+    const size_t sums = std::max({split_gemm_scratch_bytes(B, part, W), split_gemm_scratch_bytes(B, tail, W),
+                                  split_gemm_scratch_bytes(B, W, part), split_gemm_scratch_bytes(B, W, tail),
+                                  split_gemm_scratch_bytes(part, W, B), split_gemm_scratch_bytes(tail, W, B)});
     const size_t forward = split_plane_bytes(B, W) + split_plane_bytes(part, W);
     const size_t backward =
         split_plane_bytes(B, part) + split_plane_bytes(part, B) + split_plane_bytes(W, part) + split_plane_bytes(W, B);
-    return 1024 + (forward > backward ? forward : backward);
+    return 1024 + (forward > backward ? forward : backward) + sums;
   }
   size_t n0 = 0, n1 = 0, n2 = 0;
   run_tf32<RowM, ColM, kLayoutRowCol>(nullptr, nullptr, nullptr, (int)B, (int)K, (int)W, nullptr, 0, nullptr, &n0);
@@ -252,7 +257,7 @@ int smore_dot_forward_shared(const float* cand, const float* query, float* dst, 
     for (size_t k = 0; k < K; k += part) {
       const size_t n = std::min(part, K - k);
       if (int rc = split_planes(cand + k * W, W, n, W, c, nullptr, st)) return rc;
-      if (int rc = split_gemm(q, c, dst + k, K, false, B, n, W, st)) return rc;
+      if (int rc = split_gemm(q, c, dst + k, K, false, B, n, W, ws.at, st)) return rc;
     }
     return SMORE_OK;
   }
@@ -282,8 +287,8 @@ int smore_dot_backward_shared(const float* gout, const float* cand, const float*
       const size_t n = std::min(part, K - k);
       if (int rc = split_planes(gout + k, K, B, n, g, gt, st)) return rc;
       if (int rc = split_planes(cand + k * W, W, n, W, nullptr, ct, st)) return rc;
-      if (int rc = split_gemm(g, ct, g_query, W, k > 0, B, W, n, st)) return rc;
-      if (int rc = split_gemm(gt, qt, g_cand + k * W, W, false, n, W, B, st)) return rc;
+      if (int rc = split_gemm(g, ct, g_query, W, k > 0, B, W, n, ws.at, st)) return rc;
+      if (int rc = split_gemm(gt, qt, g_cand + k * W, W, false, n, W, B, ws.at, st)) return rc;
     }
     return SMORE_OK;
   }

@@ -1,9 +1,9 @@
 // fp32-accurate matrix products on the bf16 tensor cores, for dot-product scoring against a shared list.
 //
 // Every fp32 operand is split once, ahead of the product, into three bf16 planes whose sum is the operand
-// (8 + 8 + 8 significant bits); the product is the sum of the nine plane products.  A GEMM that splits its
-// operands inside the main loop repeats that work for every tile that reads them and keeps the tensor cores
-// waiting for it: 4096 x 8192 x 1000 ran at 0.49 of the bf16 rate / 9 that way.  Here the main loop only
+// (8 + 8 + 8 significant bits); the product is the sum of plane products.  A GEMM that splits its operands
+// inside the main loop repeats that work for every tile that reads them and keeps the tensor cores waiting
+// for it: the three products of a 4096 x 8192 x 1000 step took 2.09 ms that way.  Here the main loop only
 // moves bf16 tiles (TMA) and issues tcgen05.mma.
 //
 //   split_planes_kernel   fp32 [rows, cols] -> planes [3][rows][ld] and / or transposed [3][cols][ld_t]; all
@@ -11,11 +11,20 @@
 //   split_gemm_kernel     D[M, N] = A . B^T, A planes [3][M][K], B planes [3][N][K]; one 128 x 256 tile per
 //                         CTA at a time, a fixed set of CTAs walks the tiles.  Warp 0 issues the TMA loads,
 //                         warp 1 the MMAs, warps 2..9 own the result.
+//   sum_parts_kernel      adds the parts of a reduction that was cut to fill the SMs
 //
-// Precision: a tensor-memory accumulator is added to once per 16 products, with truncation.  So that this
-// does not add up over a long reduction, the accumulator holds kChunk of it only and is then added, in fp32
-// with rounding to nearest, to the running sums in the registers of warps 2..9, while the MMAs go on in a
-// second accumulator; within a chunk the products of the small planes come first.
+// Precision.  Six of the nine plane products are taken: with round-to-nearest planes the other three (second
+// by third, third by second and third by third plane) are together below 2^-25 of the operands' product, half of
+// what rounding it to fp32 may cost.  The error comes from the additions instead: a tensor-memory accumulator
+// is added to once per 16 products, with truncation, so it takes the small products first and holds kChunk = 32
+// of the reduction; it is then added, rounding to nearest, to the running sums in the registers of warps 2..9,
+// while the MMAs go on in a second accumulator; in reductions of more than kNoFlush chunks those
+// go to a tile of scratch in L2 every kFlush, so no
+// chain of additions is long.  Relative error (2-norm) of the scores of 4096 x 8192 x 1000 against 64 bits:
+// 1.5e-7 with the splitting template, 3.2e-7 with nine products in chunks of 64, 1.2e-7 like this; its
+// gradients 2.8e-7 and 4.1e-7, 3.4e-7 and 3.7e-7, 1.1e-7 and 1.2e-7.  The three products take 1.04 ms (nine
+// products in chunks of 64: 1.19; without the scratch 0.97, the gradients then at 2.1e-7 and 3.0e-7).  A reduction of
+// up to kNoFlush chunks stays in registers, which is below the template's error too.
 //
 // Every wait on an mbarrier is bounded; one that runs out sets kStatusCopyWait and lets the CTA finish.
 #include <cuda.h>
@@ -23,6 +32,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "bulk_copy.cuh"
 #include "common.cuh"
@@ -93,21 +103,24 @@ __global__ void __launch_bounds__(256)
 
 constexpr int kTileM = 128, kTileN = 256;
 constexpr int kBlockK = 32;                      // reduction per pipeline stage: 64-byte rows, 64-byte swizzle
-constexpr int kChunk = 64;                       // reduction per tensor-memory accumulator
+constexpr int kChunk = 32;                       // reduction per tensor-memory accumulator
 constexpr int kBlocksPerChunk = kChunk / kBlockK;
+constexpr int kFlush = 16, kNoFlush = 32;        // chunks whose sum is kept in registers; of a whole reduction
 constexpr int kStages = 3;
 constexpr int kPlaneA = kTileM * kBlockK * 2, kPlaneB = kTileN * kBlockK * 2;    // bytes
 constexpr int kStageBytes = 3 * (kPlaneA + kPlaneB);                             // 72 KB
-constexpr int kGemmThreads = 320;
+constexpr int kGemmThreads = 320, kResultThreads = 256;
 constexpr int kGemmSmem = kStages * kStageBytes + 1024 /* alignment */;
 
 struct GemmArgs {
   float* d;              // [M, N] row-major
   size_t ld_d;           // floats from row to row of d
+  float* spill;          // [CTAs][128 x 256], for reductions longer than kNoFlush chunks
+  float* part_sums;      // [parts][M][N] when the reduction is cut, else nullptr
   int M, N;
   bool add;              // add to d
   int k_blocks;          // stages of the whole reduction
-  int splits;            // parts the reduction is cut into; > 1: parts are added into d
+  int parts;             // parts the reduction is cut into
   int tiles_m, tiles_n;
 };
 
@@ -131,13 +144,22 @@ __device__ __forceinline__ uint64_t operand_desc(uint32_t smem) {
          ((uint64_t)4 << 61);
 }
 
+// What a product does with the buffer the tensor core reads A through: neighbours with the same A tile read it once.
+enum KeepA { kOnce, kFill, kUse, kLastUse };
+template <int KEEP>
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(idesc), "r"((unsigned)accumulate)
-      : "memory");
+#define SMORE_MMA(QUALIFIER)                                                    \
+  asm volatile(                                                                 \
+      "{\n\t.reg .pred p;\n\t"                                                  \
+      "setp.ne.b32 p, %4, 0;\n\t"                                               \
+      "tcgen05.mma.cta_group::1.kind::f16" QUALIFIER " [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem), \
+      "l"(a), "l"(b), "r"(idesc), "r"((unsigned)accumulate)                     \
+      : "memory")
+  if constexpr (KEEP == kFill) SMORE_MMA(".collector::a::fill");
+  else if constexpr (KEEP == kUse) SMORE_MMA(".collector::a::use");
+  else if constexpr (KEEP == kLastUse) SMORE_MMA(".collector::a::lastuse");
+  else SMORE_MMA("");
+#undef SMORE_MMA
 }
 
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
@@ -149,26 +171,22 @@ __device__ __forceinline__ void barrier_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bulk::smem_addr(bar)) : "memory");
 }
 
-// 32 consecutive columns of this warp's 32 tensor-memory lanes
-__device__ __forceinline__ void tmem_load32(uint32_t addr, float (&v)[32]) {
-  uint32_t r[32];
+// adds 16 consecutive columns of this warp's 32 tensor-memory lanes
+__device__ __forceinline__ void tmem_add16(uint32_t addr, float* sum) {
+  uint32_t r[16];
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]),
-        "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]),
-        "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(addr));
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+  for (int i = 0; i < 16; ++i) sum[i] += __uint_as_float(r[i]);
 }
 
-// the part of the work item `item` covers: tile and range of stages
+// the part of the work item `item` covers: tile, range of stages, part of the reduction
 struct Item {
-  int m0, n0, k_begin, k_end;
+  int m0, n0, k_begin, k_end, part;
 };
 __device__ __forceinline__ Item item_of(const GemmArgs& g, int item) {
   // parts outermost, then tiles row by row of B's tiles: CTAs that run together share operand rows in L2
@@ -177,9 +195,9 @@ __device__ __forceinline__ Item item_of(const GemmArgs& g, int item) {
   const int tn = t / g.tiles_m, tm = t - tn * g.tiles_m;
   // parts are whole chunks
   const int chunks = (g.k_blocks + kBlocksPerChunk - 1) / kBlocksPerChunk;
-  const int per = (chunks + g.splits - 1) / g.splits;
+  const int per = (chunks + g.parts - 1) / g.parts;
   return {tm * kTileM, tn * kTileN, min(g.k_blocks, part * per * kBlocksPerChunk),
-          min(g.k_blocks, (part + 1) * per * kBlocksPerChunk)};
+          min(g.k_blocks, (part + 1) * per * kBlocksPerChunk), part};
 }
 
 __global__ void __launch_bounds__(kGemmThreads, 1)
@@ -212,7 +230,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_base_sh;
-  const int items = g.tiles_m * g.tiles_n * g.splits;
+  const int items = g.tiles_m * g.tiles_n * g.parts;
 
   if (warp == 0) {
     if (lane == 0) {
@@ -254,22 +272,33 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t d = tmem + acc * kTileN;
-          bool first = true;
           for (int kb = kb0; kb < min(it.k_end, kb0 + kBlocksPerChunk); ++kb) {
             ok = wait_bar(full + stage, parity);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t a = bulk::smem_addr(ring + (size_t)stage * kStageBytes), b = a + 3 * kPlaneA;
-            // plane products, the smallest first
-            constexpr int kPa[9] = {2, 2, 1, 2, 1, 0, 1, 0, 0}, kPb[9] = {2, 1, 2, 0, 1, 2, 0, 1, 0};
-#pragma unroll
-            for (int t = 0; t < 9; ++t)
-#pragma unroll
-              for (int k = 0; k < kBlockK / 16; ++k) {
-                mma_bf16(d, operand_desc(a + kPa[t] * kPlaneA + k * 32), operand_desc(b + kPb[t] * kPlaneB + k * 32), kIdesc,
-                         !first);
-                first = false;
-              }
+            auto product = [&](auto keep, int k, int pa, int pb, bool add) {
+              mma_bf16<decltype(keep)::value>(d, operand_desc(a + pa * kPlaneA + k * 32), operand_desc(b + pb * kPlaneB + k * 32),
+                                              kIdesc, add);
+            };
+            using Once = std::integral_constant<int, kOnce>;
+            using Fill = std::integral_constant<int, kFill>;
+            using Use = std::integral_constant<int, kUse>;
+            using Last = std::integral_constant<int, kLastUse>;
+            // plane products, the large ones last; those that share an A tile next to each other: shared memory
+            // is read at 96 bytes a cycle otherwise, next to the copies that fill it at 48
+            product(Once{}, 0, 2, 0, kb > kb0);
+            product(Fill{}, 0, 1, 1, true);
+            product(Last{}, 0, 1, 0, true);
+            product(Once{}, 1, 2, 0, true);
+            product(Fill{}, 1, 1, 1, true);
+            product(Last{}, 1, 1, 0, true);
+            product(Fill{}, 0, 0, 2, true);
+            product(Last{}, 0, 0, 1, true);
+            product(Fill{}, 1, 0, 2, true);
+            product(Use{}, 1, 0, 1, true);
+            product(Last{}, 1, 0, 0, true);
+            product(Once{}, 0, 0, 0, true);
             mma_commit(empty + stage);
             if (++stage == kStages) {
               stage = 0;
@@ -295,39 +324,67 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     bool ok = true;
     for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
       const Item it = item_of(g, item);
-      float sum[kTileN / 2];
+      // the running sums leave for this CTA's tile of `spill` now and then, laid out so that a warp's
+      // accesses are contiguous
+      float4* spill = reinterpret_cast<float4*>(g.spill) + (size_t)blockIdx.x * (kTileM * kTileN / 4) + (threadIdx.x - 64);
+      const int run = (it.k_end - it.k_begin > kNoFlush * kBlocksPerChunk ? kFlush : kNoFlush) * kBlocksPerChunk;
+#pragma unroll 1
+      for (int kb1 = it.k_begin; kb1 < it.k_end && ok; kb1 += run) {
+        float sum[kTileN / 2];
 #pragma unroll
-      for (int i = 0; i < kTileN / 2; ++i) sum[i] = 0.f;
-      for (int kb0 = it.k_begin; kb0 < it.k_end; kb0 += kBlocksPerChunk) {
-        ok = wait_bar(acc_full + acc, acc_parity);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        for (int i = 0; i < kTileN / 2; ++i) sum[i] = 0.f;
+#pragma unroll 1
+        for (int kb0 = kb1; kb0 < min(it.k_end, kb1 + run); kb0 += kBlocksPerChunk) {
+          ok = wait_bar(acc_full + acc, acc_parity);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-        for (int c = 0; c < kTileN / 2; c += 32) {
-          float v[32];
-          tmem_load32(tmem + lanes + acc * kTileN + half * (kTileN / 2) + c, v);
-#pragma unroll
-          for (int i = 0; i < 32; ++i) sum[c + i] += v[i];
+          for (int c = 0; c < kTileN / 2; c += 16)
+            tmem_add16(tmem + lanes + acc * kTileN + half * (kTileN / 2) + c, sum + c);
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) barrier_arrive(acc_empty + acc);
+          if (++acc == 2) {
+            acc = 0;
+            acc_parity ^= 1u;
+          }
         }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) barrier_arrive(acc_empty + acc);
-        if (++acc == 2) {
-          acc = 0;
-          acc_parity ^= 1u;
+        const bool first = kb1 == it.k_begin;
+        if (kb1 + run < it.k_end) {
+          if (first) {
+#pragma unroll
+            for (int c = 0; c < kTileN / 2; c += 4)
+              __stcg(spill + c / 4 * kResultThreads, make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]));
+          } else {
+#pragma unroll
+            for (int c = 0; c < kTileN / 2; c += 4)
+              atomicAdd(spill + c / 4 * kResultThreads, make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]));
+          }
+          continue;
         }
-      }
-      const int m = it.m0 + quarter * 32 + lane, n0 = it.n0 + half * (kTileN / 2);
-      if (ok && m < g.M && it.k_begin < it.k_end) {
-        float* out = g.d + (size_t)m * g.ld_d + n0;
+        if (!first) {
+#pragma unroll
+          for (int c = 0; c < kTileN / 2; c += 4) {
+            const float4 v = __ldcg(spill + c / 4 * kResultThreads);
+            sum[c] += v.x;
+            sum[c + 1] += v.y;
+            sum[c + 2] += v.z;
+            sum[c + 3] += v.w;
+          }
+        }
+        const int m = it.m0 + quarter * 32 + lane, n0 = it.n0 + half * (kTileN / 2);
+        float* out = g.part_sums ? g.part_sums + ((size_t)it.part * g.M + m) * g.N + n0 : g.d + (size_t)m * g.ld_d + n0;
+        const int n = ok && m < g.M ? g.N - n0 : 0;     // columns of the result here; N is a multiple of 4
+        const bool add = g.add && !g.part_sums;
 #pragma unroll
         for (int c = 0; c < kTileN / 2; c += 4) {
-          if (n0 + c >= g.N) continue;                // N is a multiple of 4
+          if (c >= n) continue;
           const float4 v = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
-          if (g.add) atomicAdd(reinterpret_cast<float4*>(out + c), v);
+          if (add) atomicAdd(reinterpret_cast<float4*>(out + c), v);
           else *reinterpret_cast<float4*>(out + c) = v;
         }
+        __syncwarp();
       }
     }
   }
@@ -336,6 +393,26 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+  }
+}
+
+// d (+)= the parts' sums, in the order of the parts
+__global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict__ part_sums, int parts, float* __restrict__ d,
+                                                        size_t ld_d, int M, int N, bool add) {
+  const size_t n4 = (size_t)N >> 2, total = (size_t)M * n4;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+    const size_t m = i / n4, c = i - m * n4;
+    float4 s = __ldcg(reinterpret_cast<const float4*>(part_sums) + i);
+    for (int p = 1; p < parts; ++p) {
+      const float4 v = __ldcg(reinterpret_cast<const float4*>(part_sums) + p * total + i);
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    float4* out = reinterpret_cast<float4*>(d + m * ld_d) + c;
+    if (add) {
+      const float4 v = *out;
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    *out = s;
   }
 }
 
@@ -385,8 +462,25 @@ static int plane_map(CUtensorMap* map, const void* planes, size_t rows, size_t k
   return SMORE_OK;
 }
 
+// Parts of the reduction: where the tiles leave at least half of the SMs without one, as many as there are SMs
+// for, each at least kFlush chunks long.  The parts' sums then fit one tile per SM.
+static int reduction_parts(size_t M, size_t N, size_t K) {
+  const size_t tiles = ((M + kTileM - 1) / kTileM) * ((N + kTileN - 1) / kTileN);
+  const size_t flushes = (K + kChunk - 1) / kChunk / kFlush;
+  return (int)std::max<size_t>(1, std::min<size_t>((size_t)sm_count() / tiles, flushes));
+}
+
+static size_t spill_bytes(size_t K) {
+  return K > (size_t)kChunk * kNoFlush ? (size_t)sm_count() * kTileM * kTileN * sizeof(float) : 0;
+}
+
+size_t split_gemm_scratch_bytes(size_t M, size_t N, size_t K) {
+  const int parts = reduction_parts(M, N, K);
+  return spill_bytes(K) + (parts > 1 ? (parts * M * N * sizeof(float) + 1023) & ~(size_t)1023 : 0);
+}
+
 int split_gemm(const void* a_planes, const void* b_planes, float* d, size_t ld_d, bool add, size_t M, size_t N, size_t K,
-               cudaStream_t st) {
+               void* scratch, cudaStream_t st) {
   CUtensorMap map_a, map_b;
   if (int rc = plane_map(&map_a, a_planes, M, K, kTileM)) return rc;
   if (int rc = plane_map(&map_b, b_planes, N, K, kTileN)) return rc;
@@ -395,21 +489,25 @@ int split_gemm(const void* a_planes, const void* b_planes, float* d, size_t ld_d
   g.ld_d = ld_d;
   g.M = (int)M;
   g.N = (int)N;
+  g.add = add;
   g.k_blocks = (int)((K + kBlockK - 1) / kBlockK);
   g.tiles_m = (int)((M + kTileM - 1) / kTileM);
   g.tiles_n = (int)((N + kTileN - 1) / kTileN);
-  // Tiles rarely fill the last wave: cut the reduction in two where that wastes less of it (two parts added to
-  // zero give the same sum in either order; more parts, or two added to something, would not).
-  const size_t tiles = (size_t)g.tiles_m * g.tiles_n, sms = (size_t)sm_count();
-  const size_t waves1 = 2 * ((tiles + sms - 1) / sms), waves2 = (2 * tiles + sms - 1) / sms;   // in half tiles
-  g.splits = !add && waves2 < waves1 && g.k_blocks >= 16 ? 2 : 1;
-  g.add = add || g.splits > 1;
-  if (g.splits > 1 && cudaMemset2DAsync(d, ld_d * sizeof(float), 0, N * sizeof(float), M, st) != cudaSuccess)
-    return fail(SMORE_ERR_CUDA, "dot: cudaMemsetAsync failed");
+  g.parts = reduction_parts(M, N, K);
+  // (parts are rounded up to whole chunks, so the last ones may be empty)
+  const int chunks = (g.k_blocks + kBlocksPerChunk - 1) / kBlocksPerChunk, per = (chunks + g.parts - 1) / g.parts;
+  g.parts = (chunks + per - 1) / per;
+  g.spill = static_cast<float*>(scratch);
+  g.part_sums = g.parts > 1 ? reinterpret_cast<float*>(static_cast<unsigned char*>(scratch) + spill_bytes(K)) : nullptr;
   if (int rc = allow_large_smem(split_gemm_kernel, kGemmSmem)) return rc;
-  const unsigned grid = (unsigned)std::min(tiles * g.splits, sms);
+  const size_t items = (size_t)g.tiles_m * g.tiles_n * g.parts;
+  const unsigned grid = (unsigned)std::min(items, (size_t)sm_count());
   split_gemm_kernel<<<grid, kGemmThreads, kGemmSmem, st>>>(map_a, map_b, g);
-  return check_launch("split_gemm_kernel");
+  if (int rc = check_launch("split_gemm_kernel")) return rc;
+  if (g.parts == 1) return SMORE_OK;
+  const size_t ctas = std::min<size_t>((M * (N / 4) + 255) / 256, (size_t)sm_count() * 8);
+  sum_parts_kernel<<<(unsigned)ctas, 256, 0, st>>>(g.part_sums, g.parts, d, ld_d, g.M, g.N, add);
+  return check_launch("sum_parts_kernel");
 }
 
 }  // namespace smore
