@@ -97,8 +97,9 @@ __device__ __forceinline__ bool is_answer(const int64_t* ans, int n, long long i
 // A draw is a serial chain: the query's answers, the generator, the table, the search.  A CTA takes P * 256
 // consecutive positions: the answers of the queries among them are brought to shared memory once, and a
 // thread's P draws have their table reads and searches in flight together.
-// (1024 x 1024 draws by in-degree over 2.5M ids, 30 answers per query: 21.9 us with one position at
-// a time per thread, three table arrays and the search in global memory, 20.5 us like this, tables out of L2; 12.4 us with them in L2.)
+// (1024 x 1024 draws by in-degree over 2.5M ids, 30 answers per query, with one position at a time per thread,
+// three table arrays and the search in global memory -> like this: 15.1 -> 13.4 us with the tables in L2,
+// 24.3 -> 21.4 us without; P = 1 and 2 take 23.3 and 23.1 us.)
 template <int KIND, int P>
 __global__ void __launch_bounds__(kSampleThreads) sample_negatives_kernel(SampleArgs a, int64_t* __restrict__ out) {
   __shared__ int64_t staged[kStagedAnswers];

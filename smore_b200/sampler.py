@@ -53,10 +53,9 @@ class NegativeSampler(object):
             self.tables = (torch.from_numpy(prob).to(self.device), torch.from_numpy(small).to(self.device),
                            torch.from_numpy(large).to(self.device))
             if self.n_entities < 1 << 32:      # the same tables, one 16-byte entry per slot
-                entries = np.empty((self.n_entities, 2), np.int64)
-                entries[:, 0] = prob.view(np.int64)
-                entries[:, 1] = small | large << 32
-                self._entries = torch.from_numpy(entries).to(self.device)
+                prob, small, large = self.tables
+                self._entries = torch.stack((prob.view(torch.int64), small | large << 32), dim=1)
+                torch.cuda.current_stream(self.device).synchronize()      # draws may run on any stream
 
     def _draw(self, n_queries, k, csr):
         csr = csr if csr is not None else (None, None)
