@@ -97,13 +97,18 @@ __device__ __forceinline__ size_t query_offset(const RowArgs& a, int b) {
 __device__ __forceinline__ float4 ld_row4(const float4* p) { return __ldg(p); }
 
 // acc over the 4 components of one 16-byte chunk
-template <class Term>
+template <class Term, bool FAST>
+__device__ __forceinline__ void fwd1(float e0, float e1, float q0, float q1, float* acc) {
+  if constexpr (FAST) Term::fwd_fast(e0, e1, q0, q1, acc);
+  else Term::fwd(e0, e1, q0, q1, acc);
+}
+template <class Term, bool FAST = false>
 __device__ __forceinline__ void fwd4(const float4& e0, const float4& e1, const float4& q0,
                                      const float4& q1, float* acc) {
-  Term::fwd(e0.x, e1.x, q0.x, q1.x, acc);
-  Term::fwd(e0.y, e1.y, q0.y, q1.y, acc);
-  Term::fwd(e0.z, e1.z, q0.z, q1.z, acc);
-  Term::fwd(e0.w, e1.w, q0.w, q1.w, acc);
+  fwd1<Term, FAST>(e0.x, e1.x, q0.x, q1.x, acc);
+  fwd1<Term, FAST>(e0.y, e1.y, q0.y, q1.y, acc);
+  fwd1<Term, FAST>(e0.z, e1.z, q0.z, q1.z, acc);
+  fwd1<Term, FAST>(e0.w, e1.w, q0.w, q1.w, acc);
 }
 
 // POS: every q1 of the query is positive (see Term::kPositive)
@@ -582,26 +587,36 @@ __global__ void __launch_bounds__(kRowCtaThreads)
     const float* row = reinterpret_cast<const float*>(ring + (size_t)slot * row_bytes);
     const float4* row4 = reinterpret_cast<const float4*>(row);
     float acc[NB][Term::kNOut];
+    auto score = [&](auto fast_tag) {
+      constexpr bool FAST = decltype(fast_tag)::value;
 #pragma unroll
-    for (int u = 0; u < NB; ++u)
+      for (int u = 0; u < NB; ++u)
 #pragma unroll
-      for (int o = 0; o < Term::kNOut; ++o) acc[u][o] = 0.f;
-    Lanes::each(lane, a.dim,
-                [&](int j, int d4) {
-                  const float4 e0 = row4[d4];
-                  const float4 e1 = Term::kMul == 2 ? row4[dim4 + d4] : e0;
+        for (int o = 0; o < Term::kNOut; ++o) acc[u][o] = 0.f;
+      Lanes::each(lane, a.dim,
+                  [&](int j, int d4) {
+                    const float4 e0 = row4[d4];
+                    const float4 e1 = Term::kMul == 2 ? row4[dim4 + d4] : e0;
 #pragma unroll
-                  for (int u = 0; u < NB; ++u) fwd4<Term>(e0, e1, q0[u][j], q1[u][j], acc[u]);
-                },
-                [&](int d) {
-                  const float e0 = row[d], e1 = Term::kMul == 2 ? row[a.dim + d] : e0;
+                    for (int u = 0; u < NB; ++u) fwd4<Term, FAST>(e0, e1, q0[u][j], q1[u][j], acc[u]);
+                  },
+                  [&](int d) {
+                    const float e0 = row[d], e1 = Term::kMul == 2 ? row[a.dim + d] : e0;
 #pragma unroll
-                  for (int u = 0; u < NB; ++u) Term::fwd(e0, e1, t0[u], t1[u], acc[u]);
-                });
+                    for (int u = 0; u < NB; ++u) fwd1<Term, FAST>(e0, e1, t0[u], t1[u], acc[u]);
+                  });
 #pragma unroll
-    for (int u = 0; u < NB; ++u)
+      for (int u = 0; u < NB; ++u)
 #pragma unroll
-      for (int o = 0; o < Term::kNOut; ++o) acc[u][o] = warp_sum(acc[u][o]);
+        for (int o = 0; o < Term::kNOut; ++o) acc[u][o] = warp_sum(acc[u][o]);
+    };
+    score(std::integral_constant<bool, Term::kFast>{});
+    if constexpr (Term::kFast) {     // NaN operands: again, with the exact rule (every lane holds the same sums)
+      bool nan = false;
+#pragma unroll
+      for (int u = 0; u < NB; ++u) nan = nan || acc[u][0] != acc[u][0];
+      if (nan) score(std::false_type{});
+    }
     // the sums above consumed every lane's reads of the slot: it may be refilled
     __syncwarp();
     const int tn = t + stages;

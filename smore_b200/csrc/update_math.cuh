@@ -64,23 +64,22 @@ __device__ __forceinline__ void adam_elem(float g, float& p, float& m, float& v,
 // denominator's reciprocal with one correction step (P. Markstein, "Computation of elementary functions on
 // the IBM RISC System/6000 processor", 1990: with a correctly rounded reciprocal y of b, q = a y and
 // r = a - b q exact, q + r y is a / b correctly rounded).  Three instructions instead of a full division,
-// and the same value, so parameters do not depend on which kernel updated them.  That holds while b and its
-// reciprocal are far from the ends of the exponent range and a is finite; a row outside (an infinite or NaN
-// moment) divides.
+// and the same value, so parameters do not depend on which kernel updated them.  Where the quotient is not finite
+// (an infinite or NaN operand, a reciprocal that overflows) the element divides; a denominator whose reciprocal
+// would lose bits to underflow gets a NaN for it, which leads there.
 struct RowDenom {
   float denom, inv;
-  bool plain;      // divide
 };
 __device__ __forceinline__ RowDenom rowwise_denom(float v_new, const UpdateArgs& a) {
   const float d = sqrtf(v_new) / a.sqrt_bc2 + a.eps;
-  return {d, 1.0f / d, !(d > 1e-30f && d < 1e30f)};
+  return {d, d < 1e30f ? 1.0f / d : NAN};
 }
 __device__ __forceinline__ void adam_elem_rowwise(float g, float& p, float& m, const RowDenom& d, const UpdateArgs& a) {
   const float m_new = m * a.beta1 + g * a.omb1;
   const float x = a.step_size * m_new;
   const float q = x * d.inv;
-  if (d.plain || !(fabsf(q) < INFINITY)) p += x / d.denom;
-  else p += fmaf(fmaf(-q, d.denom, x), d.inv, q);
+  if (fabsf(q) < INFINITY) p += fmaf(fmaf(-q, d.denom, x), d.inv, q);
+  else p += x / d.denom;
   m = m + (m_new - m);
 }
 
