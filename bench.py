@@ -1030,7 +1030,7 @@ def kernel_table(cfg, workload, kernel_ms, notes, peak, peak_kind, fma_rate=None
     dom = max((k for k in kernels if k in alg or k in flops), key=lambda k: kernels[k]["total_ms"], default=None)
     if dom in flops:
         # tensor-core GEMM: useful flops against the measured dense bf16 rate scaled to the mode in use
-        # (TF32 issues at half the bf16 rate; the fp32 mode spends nine bf16 MMAs per product)
+        # (TF32 issues at half the bf16 rate; the fp32 mode spends six bf16 MMAs per product)
         from smore_b200 import ext_ops as _ops
         mode = _ops.dot_precision()
         try:
@@ -1038,9 +1038,9 @@ def kernel_table(cfg, workload, kernel_ms, notes, peak, peak_kind, fma_rate=None
                 bf16, src = float(json.load(f)["bf16_tflops"]), "measured bf16 burst"
         except Exception:
             bf16, src = 1590.0, "fallback bf16"
-        tpeak = bf16 / (9.0 if mode == "fp32" else 2.0)
+        tpeak = bf16 / (6.0 if mode == "fp32" else 2.0)
         roofline = {"kernel": dom, "bound": "tensor", "achieved": kernels[dom]["achieved_tflops"], "peak": round(tpeak, 1),
-                    "peak_source": "%s / %s" % (src, "9 (bf16x9 fp32 emulation)" if mode == "fp32" else "2 (tf32)"),
+                    "peak_source": "%s / %s" % (src, "6 (six bf16 products per fp32 product)" if mode == "fp32" else "2 (tf32)"),
                     "unit": "TFLOP/s", "frac": round(kernels[dom]["achieved_tflops"] / tpeak, 4), "traffic": None,
                     "timing": timing_note}
     elif dom:

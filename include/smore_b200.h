@@ -482,7 +482,7 @@ SMORE_API int smore_negative_mask(const int64_t* negatives, size_t k, const int6
  * B, K and W must be multiples of 4 (16-byte TMA strides), else SMORE_ERR_BAD_SHAPE and the
  * caller falls back to smore_dist_forward / _backward (SIMT, exact fp32 order).
  * precision: SMORE_DOT_TF32 — products of 10-bit-mantissa inputs, fp32 accumulation (error about
- * 1e-3 of sum |terms|); SMORE_DOT_FP32 — each operand split into three bf16 terms, nine MMAs per
+ * 1e-3 of sum |terms|); SMORE_DOT_FP32 — each operand split into three bf16 terms, six products per
  * product, fp32-level accuracy at a third of the rate.
  * workspace: device scratch of smore_dot_workspace_bytes(...) bytes.  smore_dot_available() is 0
  * when the library was built without a CUTLASS header tree.

@@ -8,7 +8,7 @@
 //     g_query[B, W] = g[B, K]     . cand[K, W]
 //     g_cand[K, W]  = g[B, K]^T   . query[B, W]
 // W is the row length (dim for DistMult; 2*dim for ComplEx, with the query laid out [re | im] like
-// the entity rows).  Two precisions: fp32-level (each fp32 operand split into three bf16 planes, nine bf16
+// the entity rows).  Two precisions: fp32-level (each fp32 operand split into three bf16 planes, six bf16
 // products per product: gemm_split_sm100.cu) and TF32 (10-bit mantissa products), whose kernels are CUTLASS
 // 3.x sm100 templates instantiated here: TMA loads, tcgen05.mma with TMEM accumulators, one SM per
 // 128 x 128 tile (cluster 1x1x1), fp32 in / fp32 out.
