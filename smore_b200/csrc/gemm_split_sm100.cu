@@ -22,8 +22,8 @@
 // go to a tile of scratch in L2 every kFlush, so no
 // chain of additions is long.  Relative error (2-norm) of the scores of 4096 x 8192 x 1000 against 64 bits:
 // 1.5e-7 with the splitting template, 3.2e-7 with nine products in chunks of 64, 1.2e-7 like this; its
-// gradients 2.8e-7 and 4.1e-7, 3.4e-7 and 3.7e-7, 1.1e-7 and 1.2e-7.  The three products take 1.04 ms (nine
-// products in chunks of 64: 1.19; without the scratch 0.97, the gradients then at 2.1e-7 and 3.0e-7).  A reduction of
+// gradients 2.8e-7 and 4.1e-7, 3.4e-7 and 3.7e-7, 1.1e-7 and 1.2e-7.  The three products take 0.97 ms (nine
+// products in chunks of 64: 1.19; the scratch costs 0.07, without it the gradients are at 2.1e-7 and 3.0e-7).  A reduction of
 // up to kNoFlush chunks stays in registers, which is below the template's error too.
 //
 // Every wait on an mbarrier is bounded; one that runs out sets kStatusCopyWait and lets the CTA finish.
@@ -182,6 +182,12 @@ __device__ __forceinline__ void tmem_add16(uint32_t addr, float* sum) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int i = 0; i < 16; ++i) sum[i] += __uint_as_float(r[i]);
+}
+
+__device__ __forceinline__ void store_sector(float* p, const float* v) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]),
+               "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
 }
 
 // the part of the work item `item` covers: tile, range of stages, part of the reduction
@@ -377,9 +383,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         float* out = g.part_sums ? g.part_sums + ((size_t)it.part * g.M + m) * g.N + n0 : g.d + (size_t)m * g.ld_d + n0;
         const int n = ok && m < g.M ? g.N - n0 : 0;     // columns of the result here; N is a multiple of 4
         const bool add = g.add && !g.part_sums;
+        const bool sectors = !add && ((reinterpret_cast<uintptr_t>(out) & 31) | (n & 7)) == 0;
+        // A thread owns a row of the tile, so a warp's stores go to 32 rows, and the MMAs wait for them: a whole
+        // 32-byte sector per store where rows are aligned (scores of 4096 x 8192 x 1000: 393 -> 351 us, of
+        // 4096 x 8192 x 128: 114 -> 68 us), else 16 bytes.
+        if (sectors) {
+#pragma unroll
+          for (int c = 0; c < kTileN / 2; c += 8)
+            if (c < n) store_sector(out + c, sum + c);
+        }
 #pragma unroll
         for (int c = 0; c < kTileN / 2; c += 4) {
-          if (c >= n) continue;
+          if (sectors || c >= n) continue;
           const float4 v = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
           if (add) atomicAdd(reinterpret_cast<float4*>(out + c), v);
           else *reinterpret_cast<float4*>(out + c) = v;
